@@ -826,14 +826,14 @@ __global__ void __launch_bounds__(128) k_postproc(ElemArgs<T> a, PostArgs p) {
   // Voigt (xx yy zz yz xz xy); tau and L come as (xx yy zz xy yz xz)
   const double sig[6] = {(double)(tau[0] * iJ), (double)(tau[1] * iJ), (double)(tau[2] * iJ),
                          (double)(tau[4] * iJ), (double)(tau[5] * iJ), (double)(tau[3] * iJ)};
-  T A[6], L[6], f[3];
+  T A[6], L[6];
   A[0] = T(2) * H[0] + (H[0] * H[0] + H[1] * H[1] + H[2] * H[2]);
   A[1] = T(2) * H[4] + (H[3] * H[3] + H[4] * H[4] + H[5] * H[5]);
   A[2] = T(2) * H[8] + (H[6] * H[6] + H[7] * H[7] + H[8] * H[8]);
   A[3] = H[1] + H[3] + (H[0] * H[3] + H[1] * H[4] + H[2] * H[5]);
   A[4] = H[5] + H[7] + (H[3] * H[6] + H[4] * H[7] + H[5] * H[8]);
   A[5] = H[2] + H[6] + (H[0] * H[6] + H[1] * H[7] + H[2] * H[8]);
-  sym_log1p(A, L, f);
+  sym_log1p(A, L);
   // Green strain E_ij = (H_ij + H_ji + sum_k H_ki H_kj) / 2
   auto gre = [&](int i, int j) -> double {
     return 0.5 * ((double)H[3 * i + j] + (double)H[3 * j + i] + (double)H[i] * H[j] +
