@@ -12,6 +12,7 @@
 
 #include "alya_sma.h"
 #include "sma_kernels.cuh"
+#include "sma_solo.cuh"
 #include "sma_surrogate_elem.cuh"
 
 using namespace sma;
@@ -52,9 +53,9 @@ int32_t dalloc(P** p, size_t bytes) {
 
 inline int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
-// per-element materials use compact records when a material is shared by at
-// most this many elements on average (more sharing: the material table,
-// which the caches hold)
+// with 8 lanes per element, per-element materials use compact records when a
+// material is shared by at most this many elements on average (more sharing:
+// the material table, which the caches hold)
 constexpr int COMPACT_MAX_SHARING = 4;
 
 // host restatement of sld_elmmat.f90:199-209 summed per node in element
@@ -222,6 +223,8 @@ struct sma_ctx {
   int resident = 0;                        // resident pipelined blocks per SM (lazy)
   int nelem = 0, npoin = 0;
   int64_t npad = 0, sst = 0;
+  bool solo = false;                       // one thread per element for large ranges, state tiled
+  int solo_block = SOLO_BLOCK;             // its threads per block; 0: not in this launch
   int nmate = 0;
   // element order: internal position -> user element id (colour-sorted for
   // SMA_SCATTER_COLOR, identity otherwise)
@@ -246,6 +249,7 @@ struct sma_ctx {
   MatC mat0;                               // material 0, passed by value when nmate == 1
   void* d_matx = nullptr;                  // compact per-element records (T [nelem][MATX]) or null
   bool compact = false;                    // element kernel reads d_matx instead of d_mats
+  bool many_mats = false;                  // a material per few elements (COMPACT_MAX_SHARING)
   // learned surrogate (FP32 form): weight image, statistics, eps_tr ping-pong
   // per-range element blocks (sma_set_launch_plan): plan_end[r] ends range r
   std::vector<int32_t> plan_end, plan_block;
@@ -376,7 +380,8 @@ ElemArgs<T> elem_args(sma_ctx* c, int beg, int end, bool advance, bool stepping 
   a.ts = advance ? c->d_ts : nullptr;
   a.ft = c->d_ft;
   a.npad = c->npad;
-  a.sst = c->sst;
+  a.sst = c->solo ? ST_C : c->sst;
+  a.tiled = c->solo;
   a.beg = beg;
   a.end = end;
   a.mat0 = c->mat0;
@@ -430,6 +435,42 @@ size_t elem_smem(const sma_ctx* c) {
                                         : element_smem_bytes<T>(c->block, mats);
 }
 
+template <typename T>
+ElemKernel<T> solo_kernel(const sma_ctx* c) {
+  if (c->compact) return k_element_solo<T, SOLO_COMPACT>;
+  return c->d_lmate ? k_element_solo<T, SOLO_TABLE> : k_element_solo<T, SOLO_ONE>;
+}
+
+// Elements from which a launch takes one thread per element: one warp per
+// scheduler (4 per SM).  Below that the thread-per-element kernel takes the
+// time of a single warp, 14.8 us (FP32) or 17-19 us (FP64), whatever the size,
+// and 8 lanes per element are as fast or faster: 10 k elements 11.0 / 13.5 us,
+// 19.6 k 14.6 / 19.0 us.  Above it they fall behind: 32 k 17.0 / 25.5 us
+// against 14.9 / 18.9, 250 k 78 / 146 us against 52 / 90.
+int solo_min(const sma_ctx* c) { return 128 * c->nsm; }
+
+// one element range [beg, end), by the thread-per-element kernel where the
+// context has it and the range fills the GPU with it, else 8 lanes per element
+template <typename T>
+int32_t launch_range_t(sma_ctx* c, int beg, int end, bool advance, bool stepping) {
+  if (end <= beg) return SMA_OK;
+  ElemArgs<T> a = elem_args<T>(c, beg, end, advance, stepping);
+  if (c->solo && c->solo_block && end - beg >= solo_min(c) && !a.has_grav) {
+    const int block = c->solo_block;
+    a.pf_ahead = (int64_t)c->nsm * solo_min_blocks<T>() * SOLO_BLOCK;      // one resident wave
+    solo_kernel<T>(c)<<<(unsigned)ceil_div(end - beg, block), block, solo_smem_bytes<T>(block), c->stream>>>(a);
+  } else {
+    const int64_t ntiles = ceil_div(end - beg, c->block / 8);
+    const unsigned grid = c->variant == SMA_VARIANT_PIPE
+                              ? (unsigned)std::min<int64_t>(ntiles, (int64_t)c->nsm * c->resident)
+                              : (unsigned)ntiles;
+    elem_kernel<T>(c)<<<grid, c->block, elem_smem<T>(c), c->stream>>>(a);
+  }
+  c->launches++;
+  CU(cudaGetLastError());
+  return SMA_OK;
+}
+
 // The kernel's dynamic shared-memory limit is a per-process attribute shared
 // by every context (and the no-alloc entry point): it is raised to what a
 // 256-thread block needs and never lowered.
@@ -445,6 +486,9 @@ int32_t init_element_launch_t(sma_ctx* c) {
                           (int)std::max<size_t>(smem256, 48 * 1024)));
   CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c->resident, k, block, smem));
   if (c->resident < 1) return fail(SMA_ERR_ARG, "element kernel does not fit on an SM at this block size");
+  if (c->solo)
+    CU(cudaFuncSetAttribute(solo_kernel<T>(c), cudaFuncAttributeMaxDynamicSharedMemorySize,
+                            (int)solo_smem_bytes<T>(SOLO_BLOCK)));
   return SMA_OK;
 }
 
@@ -452,6 +496,7 @@ sur::SurElemArgs sur_args(const sma_ctx* c) {
   sur::SurElemArgs s;
   s.stats = c->d_sur_stats;
   s.rcache = c->d_rcache;
+  s.rst = c->sst;
   s.xstage = c->d_xstage;
   s.clock = c->d_ts;
   s.f_margin = c->sur_margin;
@@ -524,27 +569,23 @@ int32_t sur_init_residuals(sma_ctx* c) {
 template <typename T>
 int32_t launch_plan_t(sma_ctx* c, bool advance) {
   int beg = 0;
-  const int saved = c->block;
+  const int saved = c->block, saved_solo = c->solo_block;
   for (size_t r = 0; r < c->plan_end.size(); ++r) {
     const int end = c->plan_end[r];
-    if (end > beg) {
-      c->block = c->plan_block[r];
-      ElemArgs<T> a = elem_args<T>(c, beg, end, advance && beg == 0, advance);
-      const unsigned grid = (unsigned)ceil_div(end - beg, c->block / 8);
-      elem_kernel<T>(c)<<<grid, c->block, elem_smem<T>(c), c->stream>>>(a);
-      c->launches++;
-    }
+    c->block = c->plan_block[r];
+    c->solo_block = c->block <= SOLO_BLOCK ? c->block : 0;       // wider: 8 lanes per element
+    const int32_t rc = launch_range_t<T>(c, beg, end, advance && beg == 0, advance);
+    c->block = saved;
+    c->solo_block = saved_solo;
+    if (rc) return rc;
     beg = end;
   }
-  c->block = saved;
-  CU(cudaGetLastError());
   return SMA_OK;
 }
 
 template <typename T>
 int32_t launch_elements_t(sma_ctx* c, bool advance) {
   const int nrange = (int)c->cptr.size() - 1;
-  const int epb = c->block / 8;
   if (c->resident == 0) return fail(SMA_ERR_STATE, "element launch not initialised");
   if constexpr (sizeof(T) == 4) {
     if (c->sur) {
@@ -558,20 +599,10 @@ int32_t launch_elements_t(sma_ctx* c, bool advance) {
     return launch_plan_t<T>(c, advance);
   }
   c->last_in = c->cur;
-  const ElemKernel<T> kern = elem_kernel<T>(c);
-  const size_t smem = elem_smem<T>(c);
   for (int r = 0; r < nrange; ++r) {
-    const int beg = c->cptr[r], end = c->cptr[r + 1];
-    if (end <= beg) continue;
-    ElemArgs<T> a = elem_args<T>(c, beg, end, advance && r == 0, advance);
-    const int64_t ntiles = ceil_div(end - beg, epb);
-    const unsigned grid = c->variant == SMA_VARIANT_PIPE
-                              ? (unsigned)std::min<int64_t>(ntiles, (int64_t)c->nsm * c->resident)
-                              : (unsigned)ntiles;
-    kern<<<grid, c->block, smem, c->stream>>>(a);
-    c->launches++;
+    const int32_t rc = launch_range_t<T>(c, c->cptr[r], c->cptr[r + 1], advance && r == 0, advance);
+    if (rc) return rc;
   }
-  CU(cudaGetLastError());
   return SMA_OK;
 }
 
@@ -586,16 +617,7 @@ int32_t launch_element_range_t(sma_ctx* c, int beg, int end) {
   if (end <= beg) return SMA_OK;
   if constexpr (sizeof(T) == 4)
     if (c->sur) return launch_sur_range(c, beg, end, false, false);
-  const int epb = c->block / 8;
-  ElemArgs<T> a = elem_args<T>(c, beg, end, false, false);
-  const int64_t ntiles = ceil_div(end - beg, epb);
-  const unsigned grid = c->variant == SMA_VARIANT_PIPE
-                            ? (unsigned)std::min<int64_t>(ntiles, (int64_t)c->nsm * c->resident)
-                            : (unsigned)ntiles;
-  elem_kernel<T>(c)<<<grid, c->block, elem_smem<T>(c), c->stream>>>(a);
-  c->launches++;
-  CU(cudaGetLastError());
-  return SMA_OK;
+  return launch_range_t<T>(c, beg, end, false, false);
 }
 
 // Slab plan of the pipelined element-loop boundary (atomic scatter): K
@@ -1063,17 +1085,25 @@ int32_t sma_ctx_create(const sma_mesh_desc* mesh, const sma_material_desc* mat,
   TRY(dalloc(&c->d_mats, mats.size() * sizeof(MatC)));
   TRYCU(cudaMemcpy(c->d_mats, mats.data(), mats.size() * sizeof(MatC), cudaMemcpyHostToDevice));
   c->mat0 = mats[0];
+  c->solo = run->variant == SMA_VARIANT_AUTO && c->scatter == SMA_SCATTER_ATOMIC && !c->damp &&
+            run->block <= SOLO_BLOCK && c->nelem >= solo_min(c);
+  if (c->solo) {
+    if (run->block) c->solo_block = run->block;
+    c->sst = 8 * (ceil_div(c->nelem, 32) * 32);                 // whole tiles: 3 sst values
+  }
   // Compact per-element records when the materials differ only in what the
   // record holds (moduli, eL, thresholds; the temperature rides along) and
   // are many: 64 bytes per element read into registers instead of the
   // 176-byte material staged through shared memory behind a block barrier.
   // Measured on B200: the 2.0 M-element cylinder (a material per element)
   // -15 % FP32 / -6 % FP64 element time; the 256-specimen ensemble (256
-  // materials, a table the caches hold) +16 % FP32, so a few materials keep
-  // the table.  The one-tile undamped kernel reads them; SMA_VARIANT_TABLE
-  // keeps the table.
-  if (c->d_lmate && (int64_t)c->nmate * COMPACT_MAX_SHARING >= c->nelem && c->variant == SMA_VARIANT_PLAIN &&
-      !c->damp &&
+  // materials, a table the caches hold) +16 % FP32 with 8 lanes per element,
+  // so a few materials keep the table there.  One thread per element reads a
+  // record once for 8 Gauss points: 24 specimens 82 -> 63 us FP32, 121 -> 107
+  // us FP64, so it always takes records.  The undamped kernels read them;
+  // SMA_VARIANT_TABLE keeps the table.
+  c->many_mats = (int64_t)c->nmate * COMPACT_MAX_SHARING >= c->nelem;
+  if (c->d_lmate && (c->solo || c->many_mats) && c->variant == SMA_VARIANT_PLAIN && !c->damp &&
       run->variant != SMA_VARIANT_TABLE) {
     bool shared = true;
     for (const MatC& m : mats)
@@ -1256,20 +1286,8 @@ int32_t sma_step_elements_range(sma_ctx* c, int32_t beg, int32_t end, int32_t fi
     if (c->prec == SMA_PREC_FP32 && c->sur) {
       rc = launch_sur_range(c, beg, end, first != 0, true);
     } else {
-      const int epb = c->block / 8;
-      const int64_t ntiles = ceil_div(end - beg, epb);
-      const unsigned grid = c->variant == SMA_VARIANT_PIPE
-                                ? (unsigned)std::min<int64_t>(ntiles, (int64_t)c->nsm * c->resident)
-                                : (unsigned)ntiles;
-      if (c->prec == SMA_PREC_FP32) {
-        ElemArgs<float> a = elem_args<float>(c, beg, end, first != 0, true);
-        elem_kernel<float>(c)<<<grid, c->block, elem_smem<float>(c), c->stream>>>(a);
-      } else {
-        ElemArgs<double> a = elem_args<double>(c, beg, end, first != 0, true);
-        elem_kernel<double>(c)<<<grid, c->block, elem_smem<double>(c), c->stream>>>(a);
-      }
-      c->launches++;
-      CU(cudaGetLastError());
+      rc = c->prec == SMA_PREC_FP32 ? launch_range_t<float>(c, beg, end, first != 0, true)
+                                    : launch_range_t<double>(c, beg, end, first != 0, true);
     }
   } else if (first) {
     k_advance_time<<<1, 1, 0, c->stream>>>(c->d_ts, c->d_ft);
@@ -1570,22 +1588,23 @@ static int32_t state_io(sma_ctx* c, double* host, bool in) {
   // slot TIME_N the one it reads (cur)
   void* sk = c->d_state[c->cur ^ 1];
   void* sn = c->d_state[c->cur];
+  const int64_t cs = c->solo ? ST_C : c->sst;                   // stride of a state component
   cudaError_t e = cudaSuccess;
   if (in) {
     c->last_in = -1;                       // post-processing reads TIME_N until the next loop
     e = cudaMemcpyAsync(d, host, bytes, cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) {
       if (c->prec == SMA_PREC_FP32)
-        k_state_in<float><<<grid, 256, 0, c->stream>>>(d, c->d_perm, (float*)sk, (float*)sn, c->nelem, c->sst);
+        k_state_in<float><<<grid, 256, 0, c->stream>>>(d, c->d_perm, (float*)sk, (float*)sn, c->nelem, cs, c->solo);
       else
-        k_state_in<double><<<grid, 256, 0, c->stream>>>(d, c->d_perm, (double*)sk, (double*)sn, c->nelem, c->sst);
+        k_state_in<double><<<grid, 256, 0, c->stream>>>(d, c->d_perm, (double*)sk, (double*)sn, c->nelem, cs, c->solo);
       e = cudaGetLastError();
     }
   } else {
     if (c->prec == SMA_PREC_FP32)
-      k_state_out<float><<<grid, 256, 0, c->stream>>>(d, c->d_perm, (const float*)sk, (const float*)sn, c->nelem, c->sst);
+      k_state_out<float><<<grid, 256, 0, c->stream>>>(d, c->d_perm, (const float*)sk, (const float*)sn, c->nelem, cs, c->solo);
     else
-      k_state_out<double><<<grid, 256, 0, c->stream>>>(d, c->d_perm, (const double*)sk, (const double*)sn, c->nelem, c->sst);
+      k_state_out<double><<<grid, 256, 0, c->stream>>>(d, c->d_perm, (const double*)sk, (const double*)sn, c->nelem, cs, c->solo);
     e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(host, d, bytes, cudaMemcpyDeviceToHost, c->stream);
   }
@@ -1869,7 +1888,7 @@ int64_t sma_kernel_launches(sma_ctx* c) { return c ? c->launches : 0; }
 // the element kernel's launch shape this context chose
 int32_t sma_launch_info(sma_ctx* c, int32_t* block, int32_t* variant, int32_t* compact) {
   if (!c || !block || !variant || !compact) return fail(SMA_ERR_ARG, "NULL argument");
-  *block = c->block;
+  *block = c->solo ? c->solo_block : c->block;
   *variant = c->variant;
   *compact = c->compact ? 1 : 0;
   return SMA_OK;
@@ -1968,7 +1987,7 @@ int32_t noalloc_run(unsigned char* base, int32_t nelem, int32_t npoin, const int
   T* s_timen = (T*)(base + NA_OFF_S1);
   const unsigned sgrid = (unsigned)ceil_div(8 * (int64_t)nelem, 256);
   // the caller's slot TIME_N in, slot ITER_K out: the other slot is left as it is
-  k_state_in<T><<<sgrid, 256, 0, s>>>(d_sdv, nullptr, nullptr, s_timen, nelem, sst);
+  k_state_in<T><<<sgrid, 256, 0, s>>>(d_sdv, nullptr, nullptr, s_timen, nelem, sst, 0);
   ElemArgs<T> a;
   std::memset(&a, 0, sizeof a);
   a.lnods = d_lnods;
@@ -1986,6 +2005,7 @@ int32_t noalloc_run(unsigned char* base, int32_t nelem, int32_t npoin, const int
   a.ft = nullptr;
   a.npad = NA_NPAD;
   a.sst = sst;
+  a.tiled = 0;
   a.beg = 0;
   a.end = nelem;
   a.has_grav = 0;
@@ -1995,7 +2015,7 @@ int32_t noalloc_run(unsigned char* base, int32_t nelem, int32_t npoin, const int
   const int block = 32, epb = block / 8;
   const size_t smem = element_smem_bytes<T>(block, false);      // below the 48 KB default
   k_element<T, true, false, false, true><<<(unsigned)ceil_div(nelem, epb), block, smem, s>>>(a);
-  k_state_out<T><<<sgrid, 256, 0, s>>>(d_sdv, nullptr, s_iterk, nullptr, nelem, sst);
+  k_state_out<T><<<sgrid, 256, 0, s>>>(d_sdv, nullptr, s_iterk, nullptr, nelem, sst, 0);
   CU(cudaGetLastError());
   return SMA_OK;
 }
@@ -2110,7 +2130,7 @@ extern "C" int32_t sma_set_surrogate(sma_ctx* c, const float* params, const sma_
   if (c->prec != SMA_PREC_FP32) return fail(SMA_ERR_ARG, "the surrogate runs in the FP32 precision form");
   if (c->scatter != SMA_SCATTER_ATOMIC) return fail(SMA_ERR_ARG, "the surrogate element loop scatters by atomics");
   if (c->damp) return fail(SMA_ERR_ARG, "the surrogate element loop has no Rayleigh damping");
-  if (c->d_lmate && !c->compact)
+  if (c->d_lmate && !(c->compact && c->many_mats))
     return fail(SMA_ERR_ARG, "per-element materials need compact records for the surrogate");
   if (!(gate > 0.0) || !(xs_tol >= 0.0) || !(f_margin >= 0.0) || period < 1)
     return fail(SMA_ERR_ARG, "gate > 0, xs_tol >= 0, f_margin >= 0, period >= 1");

@@ -115,12 +115,14 @@ struct ElemArgs {
   const int32_t* lmate;        // (nelem) or null
   const MatC* mats;
   const double* tempe;         // (nelem) or null
-  const T* sold;               // state TIME_N, SoA [3][sst]
+  const T* sold;               // state TIME_N: component c of Gauss point g of
+                               // element e at c sst + state_at(e, g)
   T* snew;                     // state ITER_K
   unsigned long long* cnt;
   StepTime* ts;                // non-null: advance the step time (block 0)
   const FunTab* ft;
   int64_t npad, sst;
+  int tiled;                   // state layout (state_index)
   int32_t beg, end;            // element range of this launch
   double grav[3];              // rho-scaled body force per unit mass (elfext)
   int has_grav;
@@ -130,6 +132,19 @@ struct ElemArgs {
   int64_t pf_ahead;            // elements ahead whose connectivity is prefetched to L2 (0: none)
   const T* matx;               // compact per-element records [nelem][MATX] (internal order), or null
 };
+
+// State layouts.  SoA [3][sst], Gauss point g of element e at 8 e + g: what 8
+// lanes per element read coalesced.  Tiled [elements / 32][3][8][32], sst =
+// ST_C: what one thread per element reads coalesced, a warp's 24 values a
+// thread at constant offsets.
+constexpr int ST_G = 32, ST_C = 8 * ST_G, ST_TILE = 3 * ST_C;
+__host__ __device__ __forceinline__ int64_t state_index(int tiled, int64_t e, int g) {
+  return tiled ? (e >> 5) * ST_TILE + g * ST_G + (e & 31) : 8 * e + g;
+}
+template <typename T>
+__device__ __forceinline__ int64_t state_at(const ElemArgs<T>& a, int64_t e, int g) {
+  return state_index(a.tiled, e, g);
+}
 
 // Compact per-element material record: the values a mesh whose elements
 // differ only in their moduli,
@@ -445,7 +460,7 @@ __device__ __forceinline__ void element_tile(const ElemArgs<T>& a, const T* tab,
     const T v[6] = {(T)dX[0], (T)dX[1], (T)dX[2], (T)dU[0], (T)dU[1], (T)dU[2]};
     stage_node_rows<T>(nsm, lane8, v);
   }
-  const int64_t gp = 8 * ec + lane8;
+  const int64_t gp = state_at(a, ec, lane8);
   __syncwarp();                                                  // node rows of the element
 
   // ---- phase 1, lane = Gauss point g ------------------------------------
@@ -582,7 +597,7 @@ __global__ void __launch_bounds__(NARROW ? ELEM_NARROW_BLOCK : 256,
     dX[c] = X[c] - __shfl_sync(0xffffffffu, X[c], src);
     dU[c] = U[c] - __shfl_sync(0xffffffffu, U[c], src);
   }
-  const int64_t gp = 8 * ec + lane8;
+  const int64_t gp = state_at(a, ec, lane8);
   const double xS = (double)a.sold[gp], F_AS = (double)a.sold[a.sst + gp];
   const double F_SA = (double)a.sold[2 * a.sst + gp];
   T Vn[3] = {T(0), T(0), T(0)};
@@ -665,7 +680,7 @@ __global__ void __launch_bounds__(256, (elem_min_blocks<T, true, MATS>())) k_ele
       cp_async(nd + 3 + c, a.u + c * a.npad + nid, 8);
     }
     T* ss = reinterpret_cast<T*>(st + PS::NODE_DOUBLES * 8) + 4 * lane8;
-    const int64_t gp = 8 * ec + lane8;
+    const int64_t gp = state_at(a, ec, lane8);
 #pragma unroll
     for (int c = 0; c < 3; ++c) cp_async(ss + c, a.sold + c * a.sst + gp, (int)sizeof(T));
     if constexpr (MATS) {
@@ -810,7 +825,7 @@ __global__ void __launch_bounds__(128) k_postproc(ElemArgs<T> a, PostArgs p) {
     }
     stage_node_rows<T>(nsm, lane8, v);
   }
-  const int64_t gp = 8 * ec + lane8;
+  const int64_t gp = state_at(a, ec, lane8);
   double xS = (double)a.sold[gp], F_AS = (double)a.sold[a.sst + gp];
   double F_SA = (double)a.sold[2 * a.sst + gp];
   __syncthreads();                                               // table, node rows, materials
@@ -1225,32 +1240,34 @@ __global__ void k_rayleigh(const int32_t* lnods, const double* coord, const doub
     for (int c = 0; c < 3; ++c) atomicAdd(fray + c * npad + nd[b], f[b][c]);
 }
 
-// state layout: reference (3, 8, 2, nelem) <-> SoA [3][sst] per slot; a
-// null slot pointer leaves that slot alone (not read, not written)
+// state: reference (3, 8, 2, nelem) <-> the kernels' layout (state_index) per
+// slot; a null slot pointer leaves that slot alone (not read, not written)
 template <typename T>
 __global__ void k_state_in(const double* host_layout, const int32_t* perm, T* s_iterk,
-                           T* s_timen, int64_t nelem, int64_t sst) {
+                           T* s_timen, int64_t nelem, int64_t sst, int tiled) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;   // internal gp id
   if (i >= 8 * nelem) return;
   const int64_t e = i >> 3, g = i & 7;
   const int64_t ue = perm ? perm[e] : e;
   const double* src = host_layout + 48 * ue;
+  const int64_t at = state_index(tiled, e, (int)g);
   for (int c = 0; c < 3; ++c) {
-    if (s_iterk) s_iterk[c * sst + i] = (T)src[c + 3 * g];
-    if (s_timen) s_timen[c * sst + i] = (T)src[24 + c + 3 * g];
+    if (s_iterk) s_iterk[c * sst + at] = (T)src[c + 3 * g];
+    if (s_timen) s_timen[c * sst + at] = (T)src[24 + c + 3 * g];
   }
 }
 template <typename T>
 __global__ void k_state_out(double* host_layout, const int32_t* perm, const T* s_iterk,
-                            const T* s_timen, int64_t nelem, int64_t sst) {
+                            const T* s_timen, int64_t nelem, int64_t sst, int tiled) {
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= 8 * nelem) return;
   const int64_t e = i >> 3, g = i & 7;
   const int64_t ue = perm ? perm[e] : e;
   double* dst = host_layout + 48 * ue;
+  const int64_t at = state_index(tiled, e, (int)g);
   for (int c = 0; c < 3; ++c) {
-    if (s_iterk) dst[c + 3 * g] = (double)s_iterk[c * sst + i];
-    if (s_timen) dst[24 + c + 3 * g] = (double)s_timen[c * sst + i];
+    if (s_iterk) dst[c + 3 * g] = (double)s_iterk[c * sst + at];
+    if (s_timen) dst[24 + c + 3 * g] = (double)s_timen[c * sst + at];
   }
 }
 

@@ -51,7 +51,8 @@ namespace sur {
 
 struct SurElemArgs {
   const SurStats* stats;      // the training inputs' box (lo_x, hi_x)
-  __half* rcache;             // held stress residual per Gauss point, SoA [6][sst] (NaN: none, plain law)
+  __half* rcache;             // held stress residual per Gauss point, SoA [6][rst] (NaN: none, plain law)
+  int64_t rst;
   float* xstage;              // network inputs of the due tiles, [slot][NIN][128], slot = tile / period
   const StepTime* clock;      // the step's time (its index picks the due tiles)
   float f_margin;             // distance from the transformation surfaces (loading-function units)
@@ -118,9 +119,10 @@ __global__ void __launch_bounds__(SUR_BLOCK, 6) k_element_sur(ElemArgs<float> a,
   const int nid = sur_gather(a, nsm, lane8, ec);
   float Ji[9], H[9], Jc[9];
   const float detJ = gp_kinematics<float>(nsm, lane8, Ji, H, Jc);
-  const int64_t gp = 8 * ec + lane8;
-  const double xS0 = (double)a.sold[gp], F_AS0 = (double)a.sold[a.sst + gp];
-  const double F_SA0 = (double)a.sold[2 * a.sst + gp];
+  const int64_t gp = 8 * ec + lane8;                             // held residuals
+  const int64_t gs = state_at(a, ec, lane8);                   // state
+  const double xS0 = (double)a.sold[gs], F_AS0 = (double)a.sold[a.sst + gs];
+  const double F_SA0 = (double)a.sold[2 * a.sst + gs];
   double tmp = 0.0;
   const MatC m = CMP ? compact_mat<float>(a, ec, &tmp) : a.mat0;
   if (!CMP) tmp = a.tempe ? __ldg(a.tempe + ec) : 0.0;
@@ -131,7 +133,7 @@ __global__ void __launch_bounds__(SUR_BLOCK, 6) k_element_sur(ElemArgs<float> a,
   // ---- stress from the held residual and the analytic part ------------
   float r[6];
 #pragma unroll
-  for (int c = 0; c < 6; ++c) r[c] = __half2float(s.rcache[c * a.sst + gp]);
+  for (int c = 0; c < 6; ++c) r[c] = __half2float(s.rcache[c * s.rst + gp]);
   const float Ex = 1.f / reuss_iE_f(m, xS0);
   float S[6], etr_p[6];
   {
@@ -204,12 +206,12 @@ __global__ void __launch_bounds__(SUR_BLOCK, 6) k_element_sur(ElemArgs<float> a,
     for (int c = 0; c < 6; ++c) r[c] = S[c] * rE - sp[c];
   }
   if (valid) {
-    a.snew[gp] = (float)xS;
-    a.snew[a.sst + gp] = (float)F_AS;
-    a.snew[2 * a.sst + gp] = (float)F_SA;
+    a.snew[gs] = (float)xS;
+    a.snew[a.sst + gs] = (float)F_AS;
+    a.snew[2 * a.sst + gs] = (float)F_SA;
     if (fallback)
 #pragma unroll
-      for (int c = 0; c < 6; ++c) s.rcache[c * a.sst + gp] = __float2half_rn(r[c]);
+      for (int c = 0; c < 6; ++c) s.rcache[c * s.rst + gp] = __float2half_rn(r[c]);
     if (tile % s.period == due_class(s.clock, s.period))
       sur_stage(s.xstage + (tile / s.period) * (NIN * SUR_BLOCK) + threadIdx.x, E, etr_p, tmp, xS0, fallback);
   }
@@ -269,8 +271,7 @@ __global__ void __launch_bounds__(SUR_BLOCK) k_sur_stage(ElemArgs<float> a, SurE
   green_2E<float>(H, A2);
 #pragma unroll
   for (int c = 0; c < 6; ++c) E[c] = 0.5f * A2[c];
-  const int64_t gp = 8 * ec + lane8;
-  const double xS0 = (double)a.sold[gp];
+  const double xS0 = (double)a.sold[state_at(a, ec, lane8)];
   double tmp = 0.0;
   const MatC m = CMP ? compact_mat<float>(a, ec, &tmp) : a.mat0;
   if (!CMP) tmp = a.tempe ? __ldg(a.tempe + ec) : 0.0;

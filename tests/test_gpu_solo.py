@@ -1,0 +1,152 @@
+"""The thread-per-element kernel against the 8-lane one: meshes large enough
+to take it by default, element counts that are no multiple of its warps or
+state tiles, every material layout, and Gauss points that leave its short
+forms (large strains, inverted elements)."""
+import dataclasses
+
+import numpy as np
+import pytest
+
+import alya_sma_b200 as sma
+from alya_sma_b200 import problem as P
+
+pytestmark = pytest.mark.gpu
+
+
+def _mesh(kind):
+    """20,060 elements (not a multiple of 32), above the kernel's threshold of
+    one warp per scheduler."""
+    nx, ny, nz = 59, 17, 20
+    coord, lnods = P.structured_box(nx, ny, nz, float(nx), float(ny), float(nz), 0.1, 5)
+    ne, npo = len(lnods), len(coord)
+    rng = np.random.default_rng(6)
+    props, em = P.nitinol_props(**P.NITI)[None, :], np.array([P.NITI_E_MART])
+    lmate = None
+    if kind == "one_modulus":
+        em = np.zeros(1)
+    if kind in ("compact", "table"):
+        nm = ne if kind == "compact" else 7
+        props = np.tile(P.nitinol_props(**P.NITI, C_AS=5.0, C_SA=5.0, T_ref=300.0), (nm, 1))
+        f = rng.uniform(0.9, 1.1, size=(nm, 3))
+        props[:, 0] *= f[:, 0]
+        props[:, 2] *= f[:, 1]
+        props[:, 3:5] *= f[:, 2:]
+        em = P.NITI_E_MART * f[:, 1]
+        lmate = rng.integers(0, nm, ne).astype(np.int32) if kind == "table" else np.arange(ne, dtype=np.int32)
+        if kind == "table":
+            props[:, 1] = rng.uniform(0.3, 0.35, nm)       # Poisson's ratio: no compact record
+            props[:, 14] = 0.02                             # pressure sensitivity
+    fixno = np.zeros((npo, 3), np.int32)
+    fixno[P.face_nodes(coord, 0, 0.0)] = 1
+    densi = np.full(len(props), P.NITI_DENSITY)
+    dt = 0.5 * P.critical_dt(coord, lnods, props, densi, lmate)
+    return P.Problem(coord=coord, lnods=lnods, props=props, e_mart=em, densi=densi, fixno=fixno,
+                     bcfun=np.full(npo, -1, np.int32), fun_npts=np.array([3], np.int32),
+                     fun_smooth=np.array([1], np.int32), fun_tab=P.smooth_cycle_table(1000 * dt, 700.0), lmate=lmate,
+                     tempe=None if lmate is None else rng.uniform(300.0, 310.0, ne),
+                     fext=P.face_load(coord, lnods, 0, float(nx), (1.0, 0.0, 0.0)), load_fun=0, dtime=dt, nsteps=1000)
+
+
+def _pair(prob, precision):
+    return sma.ExplicitSolid(prob, precision=precision), sma.ExplicitSolid(prob, precision=precision, variant="plain")
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("kind", ["one", "one_modulus", "compact", "table"])
+def test_steps_equal_the_8_lane_kernel(kind, precision):
+    prob = _mesh(kind)
+    u = P.prestrain(prob, 0.01)
+    a, b = _pair(prob, precision)
+    assert a.launch_info()["block"] == 64
+    for s in (a, b):
+        s.set("displ", u)
+        s.step(12)
+    # rounding in another order through 12 steps; a Gauss point within
+    # rounding of an activation test may start a step apart
+    tol = 1e-11 if precision == "fp64" else 2e-5
+    for f in ("displ", "veloc", "rhsid"):
+        x, y = a.get(f), b.get(f)
+        assert np.linalg.norm(x - y) <= tol * np.linalg.norm(y), f
+    x, y = a.state, b.state
+    assert np.linalg.norm(x - y) <= 10 * tol * np.linalg.norm(y)
+    ca, cb = a.counters(), b.counters()
+    # where the uniform prestrain is still at rest a point's loading function
+    # equals the previous step's to rounding, and rounding decides its test
+    assert cb["nr_active"] > 0 and abs(ca["nr_active"] - cb["nr_active"]) <= 0.1 * cb["nr_active"]
+    assert ca["neg_det"] == cb["neg_det"] == 0
+    # the state comes back through the reference's layout, also from a file
+    a.state = y
+    assert np.array_equal(a.state, y if precision == "fp64" else y.astype(np.float32))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("kind", ["one", "compact", "table"])
+def test_points_outside_the_short_forms(kind, precision):
+    """Strains beyond the logarithm polynomial, an inverted element and a NaN
+    displacement: the same forces and counters as the 8-lane kernel."""
+    prob = _mesh(kind)
+    rng = np.random.default_rng(3)
+    u = 0.01 * prob.coord @ rng.normal(size=(3, 3))
+    big = rng.choice(prob.npoin, 300, replace=False)
+    u[big] += 0.3 * rng.normal(size=(300, 3))               # strains of order one, some elements inverted
+    a, b = _pair(prob, precision)
+    ra, rb = a.assemble(u)["rhsid"], b.assemble(u)["rhsid"]
+    fin = np.isfinite(rb).all(axis=1)
+    assert np.array_equal(fin, np.isfinite(ra).all(axis=1))
+    # per node, relative to one element's force (E strain h^2 / 8, about 100)
+    # or what the node holds: strains of order one magnify FP32 rounding most
+    # where an element is nearly flat (1 / det F), so the bulk is compared
+    err = np.linalg.norm(ra[fin] - rb[fin], axis=1) / np.linalg.norm(rb[fin], axis=1).clip(100.0)
+    assert np.quantile(err, 0.99) < (1e-9 if precision == "fp64" else 1e-2)
+    assert np.median(err) < (1e-13 if precision == "fp64" else 1e-5)
+    ca, cb = a.counters(), b.counters()
+    assert cb["neg_det"] > 0 and abs(ca["neg_det"] - cb["neg_det"]) <= (0 if precision == "fp64" else 2)
+    assert ca["ielem_min"] == cb["ielem_min"]
+    assert abs(ca["gpdet_min"] - cb["gpdet_min"]) <= 1e-5 * abs(cb["gpdet_min"])
+    assert abs(ca["nr_active"] - cb["nr_active"]) <= 1e-3 * cb["nr_active"]
+    v = np.zeros_like(u)
+    v[7] = np.nan
+    assert np.array_equal(np.isnan(a.assemble(v)["rhsid"]), np.isnan(b.assemble(v)["rhsid"]))
+
+
+def test_ranges_checkpoints_and_plans_share_the_state(tmp_path):
+    """One context's element ranges go to either kernel (a launch plan with
+    narrow and wide blocks, slabs below the threshold), and a checkpoint moves
+    between state layouts."""
+    prob = dataclasses.replace(_mesh("one"))
+    u = P.prestrain(prob, 0.01)
+    a, b = _pair(prob, "fp64")
+    a.set_launch_plan([19_001, prob.nelem], [32, 128])
+    for s in (a, b):
+        s.set("displ", u)
+        s.step(5)
+    a.set_launch_plan([], [])
+    a.save(str(tmp_path / "c"))
+    b.load(str(tmp_path / "c"))
+    assert np.array_equal(a.state, b.state)
+    a.step(5)
+    b.step(5)
+    assert np.abs(a.get("displ") - b.get("displ")).max() <= 1e-12 * np.abs(b.get("displ")).max()
+
+
+def test_surrogate_and_postprocessing_read_the_tiled_state():
+    from alya_sma_b200 import surrogate as S
+    prob = _mesh("compact")
+    u = P.prestrain(prob, 0.01)
+    a, b = _pair(prob, "fp32")
+    base, em, spread, t = S.training_setup(prob)
+    x, y = S.generate(base, em, 512, nstep=256, seed=3, spread=spread, t_range=t, inactive_only=True)
+    net = S.Surrogate(seed=4)
+    net.fit_stats(x, y)
+    out = []
+    for s in (b, a):
+        s.set("displ", u)
+        s.step(4)
+        pp = s.postprocess()
+        s.state = b.state                                   # the same state, displacement and network
+        s.set("displ", u)
+        s.set_surrogate(net)
+        out.append((pp["caust"], s.assemble(u)["rhsid"]))
+    (p0, r0), (p1, r1) = out
+    assert np.linalg.norm(p0 - p1) <= 1e-4 * np.linalg.norm(p0)
+    assert np.abs(r0 - r1).max() <= 1e-6 * np.abs(r0).max()
