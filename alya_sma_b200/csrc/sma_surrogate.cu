@@ -115,8 +115,8 @@ int32_t sma_sur_train_step(const uint16_t* d_wb, const float* d_w, const sma_sur
   int dev = 0, nsm = 148;
   SCU(cudaGetDevice(&dev));
   SCU(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-  const int64_t tiles = (n + 127) / 128;
-  const unsigned grid = (unsigned)(tiles < nsm ? tiles : nsm);
+  const int64_t turns = (n + sur::TR_ROWS - 1) / sur::TR_ROWS;
+  const unsigned grid = (unsigned)(turns < nsm ? turns : nsm);
   sur::TrainArgs a;
   a.wb = reinterpret_cast<const __nv_bfloat16*>(d_wb);
   a.w = d_w;
@@ -126,7 +126,7 @@ int32_t sma_sur_train_step(const uint16_t* d_wb, const float* d_w, const sma_sur
   a.n = n;
   a.grad = d_grad;
   a.loss = d_loss;
-  sur::k_sur_train<<<grid, 128, smem, (cudaStream_t)stream>>>(a);
+  sur::k_sur_train<<<grid, 32 * sur::TR_WARPS, smem, (cudaStream_t)stream>>>(a);
   SCU(cudaGetLastError());
   return SMA_OK;
 }
