@@ -105,6 +105,8 @@ def lib():
         L.sma_eval_law160_tangent.argtypes = [C.c_int64, C.c_void_p, C.c_double, C.c_void_p,
                                               C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p,
                                               C.c_void_p, C.c_void_p, C.c_void_p]
+        L.sma_eval_law160_rowmajor.argtypes = L.sma_eval_law160.argtypes
+        L.sma_eval_law160_tangent_rowmajor.argtypes = L.sma_eval_law160_tangent.argtypes
         L.sma_set_nodal.argtypes = [C.c_void_p, C.c_int32, C.c_void_p]
         L.sma_step_prologue.argtypes = [C.c_void_p]
         L.sma_step_elements.argtypes = [C.c_void_p]
@@ -432,7 +434,12 @@ def eval_sld_stress_model_160(props, gpgdi, gpsdv, gptmp=None, flagt=0, e_mart=0
     F = torch.as_tensor(np.asarray(gpgdi) if not torch.is_tensor(gpgdi) else gpgdi,
                         dtype=torch.float64, device=dev)
     n = F.shape[0]
-    Fc = F.reshape(n, 3, 3).transpose(1, 2).contiguous()          # column-major per point
+    # row-major per point as given; a transposed view is column-major in memory
+    F = F.reshape(n, 3, 3)
+    Fc = F.transpose(1, 2)
+    row = not Fc.is_contiguous()
+    if row:
+        Fc = F.contiguous()
     S0 = torch.as_tensor(np.asarray(gpsdv) if not torch.is_tensor(gpsdv) else gpsdv,
                          dtype=torch.float64, device=dev).reshape(n, 3).contiguous()
     T = None
@@ -445,17 +452,17 @@ def eval_sld_stress_model_160(props, gpgdi, gpsdv, gptmp=None, flagt=0, e_mart=0
     pr = np.ascontiguousarray(props, dtype=np.float64).reshape(18)
     if flagt == 1:
         D = torch.empty((n, 81), dtype=torch.float64, device=dev)
-        _check(lib().sma_eval_law160_tangent(n, _p(pr), float(e_mart), Fc.data_ptr(),
-                                             None if T is None else T.data_ptr(), S0.data_ptr(),
-                                             S1.data_ptr(), P.data_ptr(), D.data_ptr(),
-                                             fl.data_ptr(), torch.cuda.current_stream().cuda_stream))
+        call = lib().sma_eval_law160_tangent_rowmajor if row else lib().sma_eval_law160_tangent
+        _check(call(n, _p(pr), float(e_mart), Fc.data_ptr(), None if T is None else T.data_ptr(),
+                    S0.data_ptr(), S1.data_ptr(), P.data_ptr(), D.data_ptr(), fl.data_ptr(),
+                    torch.cuda.current_stream().cuda_stream))
         torch.cuda.current_stream().synchronize()
         gpdds = D.reshape(n, 3, 3, 3, 3).permute(0, 4, 3, 2, 1)     # column-major (i,j,k,l)
         return P.reshape(n, 3, 3).transpose(1, 2), S1, fl, gpdds
-    _check(lib().sma_eval_law160(n, _p(pr), float(e_mart), Fc.data_ptr(),
-                                 None if T is None else T.data_ptr(), S0.data_ptr(),
-                                 S1.data_ptr(), P.data_ptr(), fl.data_ptr(), PREC[precision],
-                                 torch.cuda.current_stream().cuda_stream))
+    call = lib().sma_eval_law160_rowmajor if row else lib().sma_eval_law160
+    _check(call(n, _p(pr), float(e_mart), Fc.data_ptr(), None if T is None else T.data_ptr(),
+                S0.data_ptr(), S1.data_ptr(), P.data_ptr(), fl.data_ptr(), PREC[precision],
+                torch.cuda.current_stream().cuda_stream))
     torch.cuda.current_stream().synchronize()
     gpstr = P.reshape(n, 3, 3).transpose(1, 2)
     return gpstr, S1, fl

@@ -1894,35 +1894,68 @@ int32_t sma_launch_info(sma_ctx* c, int32_t* block, int32_t* variant, int32_t* c
   return SMA_OK;
 }
 
-int32_t sma_eval_law160(int64_t n, const double* props, double e_mart, const double* d_F,
-                        const double* d_tmp, const double* d_sdv_old, double* d_sdv_new,
-                        double* d_pk2, int32_t* d_nr_flag, int32_t precision, void* stream) {
+}  // extern "C"
+
+namespace {
+
+int32_t eval_law(bool row, int64_t n, const double* props, double e_mart, const double* d_F, const double* d_tmp,
+                 const double* d_sdv_old, double* d_sdv_new, double* d_pk2, int32_t* d_nr_flag, int32_t precision,
+                 void* stream) {
   if (n < 0) return fail(SMA_ERR_ARG, "n < 0");
   if (n == 0) return SMA_OK;
   if (!props || !d_F || !d_sdv_old || !d_sdv_new || !d_pk2) return fail(SMA_ERR_ARG, "NULL argument");
   if (precision != SMA_PREC_FP64 && precision != SMA_PREC_FP32) return fail(SMA_ERR_ARG, "precision");
   const MatC m = make_mat(props, e_mart, 1.0);
   cudaStream_t s = (cudaStream_t)stream;
-  const unsigned grid = (unsigned)ceil_div(n, 128);
-  if (precision == SMA_PREC_FP32)
-    k_law_batch<float><<<grid, 128, 0, s>>>(n, m, d_F, d_tmp, d_sdv_old, d_sdv_new, d_pk2, d_nr_flag);
-  else
-    k_law_batch<double><<<grid, 128, 0, s>>>(n, m, d_F, d_tmp, d_sdv_old, d_sdv_new, d_pk2, d_nr_flag);
+  const unsigned grid = (unsigned)ceil_div(n, LAW_BLOCK);
+  auto k = precision == SMA_PREC_FP32 ? (row ? k_law_batch<float, true> : k_law_batch<float, false>)
+                                      : (row ? k_law_batch<double, true> : k_law_batch<double, false>);
+  k<<<grid, LAW_BLOCK, 0, s>>>(n, m, d_F, d_tmp, d_sdv_old, d_sdv_new, d_pk2, d_nr_flag);
   CU(cudaGetLastError());
   return SMA_OK;
+}
+
+int32_t eval_tangent(bool row, int64_t n, const double* props, double e_mart, const double* d_F, const double* d_tmp,
+                     const double* d_sdv_old, double* d_sdv_new, double* d_pk2, double* d_dds, int32_t* d_nr_flag,
+                     void* stream) {
+  if (n < 0) return fail(SMA_ERR_ARG, "n < 0");
+  if (n == 0) return SMA_OK;
+  if (!props || !d_F || !d_sdv_old || !d_sdv_new || !d_pk2 || !d_dds) return fail(SMA_ERR_ARG, "NULL argument");
+  const MatC m = make_mat(props, e_mart, 1.0);
+  auto k = row ? k_law_tangent<true> : k_law_tangent<false>;
+  k<<<(unsigned)ceil_div(n, TAN_PTS), LAW_BLOCK, sizeof(TanSmem), (cudaStream_t)stream>>>(
+      n, m, d_F, d_tmp, d_sdv_old, d_sdv_new, d_pk2, d_dds, d_nr_flag);   // below the 48 KB default
+  CU(cudaGetLastError());
+  return SMA_OK;
+}
+static_assert(sizeof(TanSmem) <= 48 * 1024, "tangent kernel's shared memory");
+
+}  // namespace
+
+extern "C" {
+
+int32_t sma_eval_law160(int64_t n, const double* props, double e_mart, const double* d_F,
+                        const double* d_tmp, const double* d_sdv_old, double* d_sdv_new,
+                        double* d_pk2, int32_t* d_nr_flag, int32_t precision, void* stream) {
+  return eval_law(false, n, props, e_mart, d_F, d_tmp, d_sdv_old, d_sdv_new, d_pk2, d_nr_flag, precision, stream);
+}
+
+int32_t sma_eval_law160_rowmajor(int64_t n, const double* props, double e_mart, const double* d_F,
+                                 const double* d_tmp, const double* d_sdv_old, double* d_sdv_new,
+                                 double* d_pk2, int32_t* d_nr_flag, int32_t precision, void* stream) {
+  return eval_law(true, n, props, e_mart, d_F, d_tmp, d_sdv_old, d_sdv_new, d_pk2, d_nr_flag, precision, stream);
 }
 
 int32_t sma_eval_law160_tangent(int64_t n, const double* props, double e_mart, const double* d_F,
                                 const double* d_tmp, const double* d_sdv_old, double* d_sdv_new,
                                 double* d_pk2, double* d_dds, int32_t* d_nr_flag, void* stream) {
-  if (n < 0) return fail(SMA_ERR_ARG, "n < 0");
-  if (n == 0) return SMA_OK;
-  if (!props || !d_F || !d_sdv_old || !d_sdv_new || !d_pk2 || !d_dds) return fail(SMA_ERR_ARG, "NULL argument");
-  const MatC m = make_mat(props, e_mart, 1.0);
-  k_law_tangent<<<(unsigned)ceil_div(n, 128), 128, 0, (cudaStream_t)stream>>>(
-      n, m, d_F, d_tmp, d_sdv_old, d_sdv_new, d_pk2, d_dds, d_nr_flag);
-  CU(cudaGetLastError());
-  return SMA_OK;
+  return eval_tangent(false, n, props, e_mart, d_F, d_tmp, d_sdv_old, d_sdv_new, d_pk2, d_dds, d_nr_flag, stream);
+}
+
+int32_t sma_eval_law160_tangent_rowmajor(int64_t n, const double* props, double e_mart, const double* d_F,
+                                         const double* d_tmp, const double* d_sdv_old, double* d_sdv_new,
+                                         double* d_pk2, double* d_dds, int32_t* d_nr_flag, void* stream) {
+  return eval_tangent(true, n, props, e_mart, d_F, d_tmp, d_sdv_old, d_sdv_new, d_pk2, d_dds, d_nr_flag, stream);
 }
 
 }  // extern "C"

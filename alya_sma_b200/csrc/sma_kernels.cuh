@@ -1292,46 +1292,92 @@ __global__ void k_scatter_rows(double* f, int64_t npad, int64_t npoin, int32_t n
 }
 
 // ---------------------------------------------------------------------------
-// batched law (material-plugin boundary): F column-major (9n) -> PK2 (9n)
+// batched law (material-plugin boundary): F (9n) -> PK2 (9n), each point's
+// tensor column-major (the reference's layout) or, ROW, row-major (F[9 g + 3 i
+// + j] = F(i, j)).  A block's 9-value tensors are one contiguous range: they
+// pass through shared memory so that global accesses are consecutive across
+// lanes (a lane's own 9 values lie 72 bytes from its neighbour's).
+// Bound by memory and the latency of a point's chain: 64 registers, so 32
+// warps per SM, beat 94 without spills (3.0 M points: FP32 138 -> 106 us,
+// FP64 156 -> 118; 91 us is the time of its 196 bytes per point).  Before, with
+// a transposed copy of F (91 us) and direct loads and stores, 150 us.
 // ---------------------------------------------------------------------------
-template <typename T>
-__global__ void k_law_batch(int64_t n, MatC mat, const double* F, const double* tmp,
-                            const double* sdv_old, double* sdv_new, double* pk2,
-                            int32_t* nr_flag) {
-  const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= n) return;
-  const double* Fg = F + 9 * g;
-  T H[9];
+constexpr int LAW_BLOCK = 128;
+
+// a full block's W values per thread, all loads in flight at once; the last
+// block's remainder one by one
+template <int W>
+__device__ __forceinline__ void block_load(double* sm, const double* src, int64_t first, int64_t n) {
+  src += first * W;
+  if (first + LAW_BLOCK <= n) {
+    double v[W];
 #pragma unroll
-  for (int i = 0; i < 3; ++i)
+    for (int k = 0; k < W; ++k) v[k] = src[k * LAW_BLOCK + threadIdx.x];
 #pragma unroll
-    for (int j = 0; j < 3; ++j) H[3 * i + j] = (T)(Fg[i + 3 * j] - (i == j ? 1.0 : 0.0));
-  double xS = sdv_old[3 * g], F_AS = sdv_old[3 * g + 1], F_SA = sdv_old[3 * g + 2];
-  T tau[6];
-  const int fl = law160_tau<T>(mat, H, tmp ? tmp[g] : 0.0, xS, F_AS, F_SA, tau);
-  sdv_new[3 * g] = xS;
-  sdv_new[3 * g + 1] = F_AS;
-  sdv_new[3 * g + 2] = F_SA;
-  // S = F^-1 tau F^-T (eval_sld_stress_model_160, :159-168)
-  T Fm[9], Fi[9];
+    for (int k = 0; k < W; ++k) sm[k * LAW_BLOCK + threadIdx.x] = v[k];
+  } else {
+    for (int k = threadIdx.x; k < (int)(n - first) * W; k += LAW_BLOCK) sm[k] = src[k];
+  }
+}
+template <int W>
+__device__ __forceinline__ void block_store(double* dst, const double* sm, int64_t first, int64_t n) {
+  dst += first * W;
+  if (first + LAW_BLOCK <= n) {
 #pragma unroll
-  for (int k = 0; k < 9; ++k) Fm[k] = H[k];
-  Fm[0] += T(1); Fm[4] += T(1); Fm[8] += T(1);
-  inv3(Fm, Fi);
-  const T tf[9] = {tau[0], tau[3], tau[5], tau[3], tau[1], tau[4], tau[5], tau[4], tau[2]};
-  T Wt[9];                                   // Fi tau
+    for (int k = 0; k < W; ++k) dst[k * LAW_BLOCK + threadIdx.x] = sm[k * LAW_BLOCK + threadIdx.x];
+  } else {
+    for (int k = threadIdx.x; k < (int)(n - first) * W; k += LAW_BLOCK) dst[k] = sm[k];
+  }
+}
+
+template <typename T, bool ROW>
+__global__ void __launch_bounds__(LAW_BLOCK, 8) k_law_batch(int64_t n, MatC mat, const double* F, const double* tmp,
+                                                         const double* sdv_old, double* sdv_new, double* pk2,
+                                                         int32_t* nr_flag) {
+  __shared__ double sf[9 * LAW_BLOCK], ss[3 * LAW_BLOCK];
+  const int64_t first = (int64_t)blockIdx.x * LAW_BLOCK;
+  const int64_t g = first + threadIdx.x;
+  block_load<9>(sf, F, first, n);
+  block_load<3>(ss, sdv_old, first, n);
+  __syncthreads();
+  double* Fg = sf + 9 * threadIdx.x;
+  double* sg = ss + 3 * threadIdx.x;
+  if (g < n) {
+    T H[9];
 #pragma unroll
-  for (int i = 0; i < 3; ++i)
+    for (int i = 0; i < 3; ++i)
 #pragma unroll
-    for (int l = 0; l < 3; ++l)
-      Wt[3 * i + l] = Fi[3 * i + 0] * tf[0 + l] + Fi[3 * i + 1] * tf[3 + l] + Fi[3 * i + 2] * tf[6 + l];
+      for (int j = 0; j < 3; ++j) H[3 * i + j] = (T)(Fg[ROW ? 3 * i + j : i + 3 * j] - (i == j ? 1.0 : 0.0));
+    double xS = sg[0], F_AS = sg[1], F_SA = sg[2];
+    T tau[6];
+    const int fl = law160_tau<T>(mat, H, tmp ? tmp[g] : 0.0, xS, F_AS, F_SA, tau);
+    sg[0] = xS;
+    sg[1] = F_AS;
+    sg[2] = F_SA;
+    // S = F^-1 tau F^-T (eval_sld_stress_model_160, :159-168)
+    T Fm[9], Fi[9];
 #pragma unroll
-  for (int i = 0; i < 3; ++i)
+    for (int k = 0; k < 9; ++k) Fm[k] = H[k];
+    Fm[0] += T(1); Fm[4] += T(1); Fm[8] += T(1);
+    inv3(Fm, Fi);
+    const T tf[9] = {tau[0], tau[3], tau[5], tau[3], tau[1], tau[4], tau[5], tau[4], tau[2]};
+    T Wt[9];                                 // Fi tau
 #pragma unroll
-    for (int j = 0; j < 3; ++j)
-      pk2[9 * g + i + 3 * j] = (double)(Wt[3 * i + 0] * Fi[3 * j + 0] + Wt[3 * i + 1] * Fi[3 * j + 1] +
-                                        Wt[3 * i + 2] * Fi[3 * j + 2]);
-  if (nr_flag) nr_flag[g] = fl;
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int l = 0; l < 3; ++l)
+        Wt[3 * i + l] = Fi[3 * i + 0] * tf[0 + l] + Fi[3 * i + 1] * tf[3 + l] + Fi[3 * i + 2] * tf[6 + l];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+        Fg[i + 3 * j] = (double)(Wt[3 * i + 0] * Fi[3 * j + 0] + Wt[3 * i + 1] * Fi[3 * j + 1] +
+                                 Wt[3 * i + 2] * Fi[3 * j + 2]);
+    if (nr_flag) nr_flag[g] = fl;
+  }
+  __syncthreads();
+  block_store<9>(pk2, sf, first, n);
+  block_store<3>(sdv_new, ss, first, n);
 }
 
 // ---------------------------------------------------------------------------
@@ -1345,104 +1391,162 @@ __global__ void k_law_batch(int64_t n, MatC mat, const double* F, const double* 
 // are symmetric, so the tangent is carried as a 6 x 6 matrix on
 // (xx yy zz xy yz xz) and expanded to the reference's (3,3,3,3) on output:
 // dds[i + 3j + 9k + 27l + 81g].
+//
+// 8 lanes per point: lanes 0-5 evaluate the perturbed stresses, lane 6 the
+// unperturbed one, all at once; lane s then owns pair s of the pull-back G =
+// Q X Q^T, its rows of X and Q passing through shared memory, and the
+// expansion to 81 values happens as the block stores them in order.  Bound by
+// instruction issue (61 %) and the FP64 pipe (45 %).  One thread per point,
+// with its matrices in local memory and 648-byte strides between lanes'
+// stores, took 101 us for 131 k points; 63 us now (80 registers, 24 warps per
+// SM; 96 registers 67, 64 registers 64).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ int voigt6(int i, int j) {
   return i == j ? i : (i + j == 1 ? 3 : (i + j == 3 ? 4 : 5));
 }
+// the pair (i, j) of v, by select instead of a table (v varies over lanes)
 __device__ __forceinline__ void voigt6_pair(int v, int& i, int& j) {
   i = v < 3 ? v : (v == 4 ? 1 : 0);
   j = v < 3 ? v : (v == 3 ? 1 : 2);
 }
 
-__global__ void __launch_bounds__(128) k_law_tangent(int64_t n, MatC mat, const double* F,
-                                                     const double* tmp, const double* sdv_old,
-                                                     double* sdv_new, double* pk2, double* dds,
-                                                     int32_t* nr_flag) {
-  const int64_t g = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (g >= n) return;
+constexpr int TAN_PTS = LAW_BLOCK / 8;                           // points of a block
+struct TanSmem {
+  double F[TAN_PTS][9];                                          // in, then PK2 out
+  double s[TAN_PTS][3];                                          // state in, then out
+  double tau[TAN_PTS][6];
+  double X[TAN_PTS][6][6], Q[TAN_PTS][6][6];
+  double G[TAN_PTS][36];                                         // the tangent on pairs, G[6 s + t]
+  double Fi[TAN_PTS][9];                                         // F^-1
+};
+
+template <bool ROW>
+__global__ void __launch_bounds__(LAW_BLOCK, 6) k_law_tangent(int64_t n, MatC mat, const double* F, const double* tmp,
+                                                           const double* sdv_old, double* sdv_new, double* pk2,
+                                                           double* dds, int32_t* nr_flag) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  TanSmem& sm = *reinterpret_cast<TanSmem*>(smem_raw);
+  const int lane8 = threadIdx.x & 7, lp = threadIdx.x >> 3;
+  const int64_t first = (int64_t)blockIdx.x * TAN_PTS;
+  const int npt = (int)min((int64_t)TAN_PTS, n - first);
+  for (int k = threadIdx.x; k < 9 * npt; k += LAW_BLOCK) (&sm.F[0][0])[k] = F[9 * first + k];
+  for (int k = threadIdx.x; k < 3 * npt; k += LAW_BLOCK) (&sm.s[0][0])[k] = sdv_old[3 * first + k];
+  __syncthreads();
+  // points past n repeat the block's last one and store nothing
+  const int q = min(lp, npt - 1);
+  const int64_t g = first + q;
+  const bool live = lp < npt;
   const double eps = 1.0e-5;
-  const double* Fg = F + 9 * g;
-  double Fm[9], H[9];                                        // Fm[3i+j] = F(i, j)
+  double Fm[9], H[9];                                            // Fm[3i+j] = F(i, j)
+#pragma unroll
   for (int i = 0; i < 3; ++i)
+#pragma unroll
     for (int j = 0; j < 3; ++j) {
-      Fm[3 * i + j] = Fg[i + 3 * j];
+      Fm[3 * i + j] = sm.F[q][ROW ? 3 * i + j : i + 3 * j];
       H[3 * i + j] = Fm[3 * i + j] - (i == j ? 1.0 : 0.0);
     }
-  const double tg = tmp ? tmp[g] : 0.0;
-  const double xs0 = sdv_old[3 * g], fas0 = sdv_old[3 * g + 1], fsa0 = sdv_old[3 * g + 2];
-  double xS = xs0, F_AS = fas0, F_SA = fsa0, tau[6];
-  const int fl = law160_tau<double>(mat, H, tg, xS, F_AS, F_SA, tau);
-  sdv_new[3 * g] = xS;
-  sdv_new[3 * g + 1] = F_AS;
-  sdv_new[3 * g + 2] = F_SA;
-  if (nr_flag) nr_flag[g] = fl;
-
-  // X[p][v]: d tau_v for the perturbation pair p, minus the Eq. 68 term
-  double X[6][6];
-  for (int p = 0; p < 6; ++p) {
-    int i, j;
-    voigt6_pair(p, i, j);
-    double Hp[9];
-    for (int r = 0; r < 3; ++r)
-      for (int c = 0; c < 3; ++c) {
-        const double a = (r == i ? Fm[3 * j + c] : 0.0) + (r == j ? Fm[3 * i + c] : 0.0);
-        Hp[3 * r + c] = H[3 * r + c] + 0.5 * eps * a;
-      }
-    double xs = xs0, fas = fas0, fsa = fsa0, tp[6];
-    law160_tau<double>(mat, Hp, tg, xs, fas, fsa, tp);
-    for (int v = 0; v < 6; ++v) {
-      int c, d;
-      voigt6_pair(v, c, d);
-      const double corr = (i == c ? tau[voigt6(d, j)] : 0.0) + (c == j ? tau[voigt6(i, d)] : 0.0) +
-                          (i == d ? tau[voigt6(c, j)] : 0.0) + (d == j ? tau[voigt6(i, c)] : 0.0);
-      X[p][v] = (tp[v] - tau[v]) / eps - 0.5 * corr;
-    }
+  int pi, pj;                                                    // the lane's pair
+  voigt6_pair(lane8 < 6 ? lane8 : 0, pi, pj);
+  // lanes 0-5 perturb: rows pi and pj of H gain 0.5 eps times rows pj, pi of F
+  const double h = lane8 < 6 ? 0.5 * eps : 0.0;
+  double di[3], dj[3];
+#pragma unroll
+  for (int m = 0; m < 3; ++m) {
+    di[m] = pi == m ? 1.0 : 0.0;
+    dj[m] = pj == m ? 1.0 : 0.0;
   }
-
-  // pull-back: G = Q X Q^T with Q[s][w] = sum over (m, n) of pair w of
-  // F^-1(i, m) F^-1(j, n), (i, j) the pair s
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    const double ri = h * sm.F[q][ROW ? 3 * pi + c : pi + 3 * c], rj = h * sm.F[q][ROW ? 3 * pj + c : pj + 3 * c];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) H[3 * r + c] += di[r] * rj + dj[r] * ri;
+  }
+  double xS = sm.s[q][0], F_AS = sm.s[q][1], F_SA = sm.s[q][2], tau[6];
+  const int fl = law160_tau<double>(mat, H, tmp ? tmp[g] : 0.0, xS, F_AS, F_SA, tau);
   double Fi[9];
   inv3(Fm, Fi);
-  double Q[6][6];
-  for (int s = 0; s < 6; ++s) {
-    int i, j;
-    voigt6_pair(s, i, j);
+  if (lane8 == 6 && live) {
+#pragma unroll
+    for (int k = 0; k < 9; ++k) sm.Fi[lp][k] = Fi[k];
+#pragma unroll
+    for (int v = 0; v < 6; ++v) sm.tau[lp][v] = tau[v];
+    if (nr_flag) nr_flag[g] = fl;
+  }
+  __syncthreads();                                               // tau, F^-1; F and the state have been read
+  if (lane8 == 6 && live) {
+    sm.s[lp][0] = xS;
+    sm.s[lp][1] = F_AS;
+    sm.s[lp][2] = F_SA;
+    // S = F^-1 tau F^-T (eval_sld_stress_model_160, :159-168)
+    const double tf[9] = {tau[0], tau[3], tau[5], tau[3], tau[1], tau[4], tau[5], tau[4], tau[2]};
+    double Wt[9];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int l = 0; l < 3; ++l)
+        Wt[3 * i + l] = Fi[3 * i] * tf[l] + Fi[3 * i + 1] * tf[3 + l] + Fi[3 * i + 2] * tf[6 + l];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+        sm.F[lp][i + 3 * j] = Wt[3 * i] * Fi[3 * j] + Wt[3 * i + 1] * Fi[3 * j + 1] + Wt[3 * i + 2] * Fi[3 * j + 2];
+  }
+  double Qr[6];                                                  // row lane8 of Q: Q[s][w] = sum over (m, n) of
+  if (lane8 < 6 && live) {                                       // pair w of F^-1(i, m) F^-1(j, n)
+    double fi[3], fj[3], ti[3], tj[3];                           // rows i, j of F^-1 and of the stress
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      fi[m] = sm.Fi[lp][3 * pi + m];
+      fj[m] = sm.Fi[lp][3 * pj + m];
+      ti[m] = sm.tau[lp][voigt6(pi, m)];
+      tj[m] = sm.tau[lp][voigt6(pj, m)];
+    }
+#pragma unroll
     for (int w = 0; w < 6; ++w) {
-      int m, nn;
-      voigt6_pair(w, m, nn);
-      Q[s][w] = Fi[3 * i + m] * Fi[3 * j + nn] + (m != nn ? Fi[3 * i + nn] * Fi[3 * j + m] : 0.0);
+      constexpr int wm[6] = {0, 1, 2, 0, 1, 0}, wn[6] = {0, 1, 2, 1, 2, 2};
+      const int m = wm[w], nn = wn[w];
+      Qr[w] = fi[m] * fj[nn] + (m != nn ? fi[nn] * fj[m] : 0.0);
+      sm.Q[lp][lane8][w] = Qr[w];
+      // X[pair][w]: d tau_w minus the Eq. 68 term
+      const double corr = di[m] * tj[nn] + dj[m] * ti[nn] + di[nn] * tj[m] + dj[nn] * ti[m];
+      sm.X[lp][lane8][w] = (tau[w] - sm.tau[lp][w]) * 1.0e5 - 0.5 * corr;   // 1 / eps
     }
   }
-  double Y[6][6];                                            // Y = X Q^T
-  for (int w = 0; w < 6; ++w)
-    for (int t = 0; t < 6; ++t) {
-      double acc = 0.0;
-      for (int u = 0; u < 6; ++u) acc += X[w][u] * Q[t][u];
-      Y[w][t] = acc;
+  __syncwarp();
+  if (lane8 < 6 && live) {
+    // column t = lane8 of G = Q (X Q^T)
+    double Y[6];
+#pragma unroll
+    for (int w = 0; w < 6; ++w) {
+      Y[w] = 0.0;
+#pragma unroll
+      for (int u = 0; u < 6; ++u) Y[w] += sm.X[lp][w][u] * Qr[u];
     }
-  double* out = dds + 81 * g;
-  for (int s = 0; s < 6; ++s)
-    for (int t = 0; t < 6; ++t) {
+#pragma unroll
+    for (int s = 0; s < 6; ++s) {
       double acc = 0.0;
-      for (int w = 0; w < 6; ++w) acc += Q[s][w] * Y[w][t];
-      int i, j, k, l;
-      voigt6_pair(s, i, j);
-      voigt6_pair(t, k, l);
-      out[i + 3 * j + 9 * k + 27 * l] = acc;
-      out[j + 3 * i + 9 * k + 27 * l] = acc;
-      out[i + 3 * j + 9 * l + 27 * k] = acc;
-      out[j + 3 * i + 9 * l + 27 * k] = acc;
+#pragma unroll
+      for (int w = 0; w < 6; ++w) acc += sm.Q[lp][s][w] * Y[w];
+      sm.G[lp][6 * s + lane8] = acc;
     }
-
-  // S = F^-1 tau F^-T (eval_sld_stress_model_160, :159-168)
-  const double tf[9] = {tau[0], tau[3], tau[5], tau[3], tau[1], tau[4], tau[5], tau[4], tau[2]};
-  for (int i = 0; i < 3; ++i)
-    for (int j = 0; j < 3; ++j) {
-      double acc = 0.0;
-      for (int k = 0; k < 3; ++k)
-        for (int l = 0; l < 3; ++l) acc += Fi[3 * i + k] * Fi[3 * j + l] * tf[3 * k + l];
-      pk2[9 * g + i + 3 * j] = acc;
-    }
+  }
+  __syncthreads();
+  // a warp stores its 4 points, component r of dds from entry at(r) of G
+  {
+    const int lane = threadIdx.x & 31, p0 = threadIdx.x >> 5 << 2;
+    auto at = [](int r) { return 6 * voigt6(r % 3, r / 3 % 3) + voigt6(r / 9 % 3, r / 27); };
+    const int a0 = at(lane), a1 = at(lane + 32), a2 = lane < 17 ? at(lane + 64) : 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (p0 + k < npt) {
+        double* o = dds + 81 * (first + p0 + k) + lane;
+        o[0] = sm.G[p0 + k][a0];
+        o[32] = sm.G[p0 + k][a1];
+        if (lane < 17) o[64] = sm.G[p0 + k][a2];
+      }
+  }
+  for (int k = threadIdx.x; k < 9 * npt; k += LAW_BLOCK) pk2[9 * first + k] = (&sm.F[0][0])[k];
+  for (int k = threadIdx.x; k < 3 * npt; k += LAW_BLOCK) sdv_new[3 * first + k] = (&sm.s[0][0])[k];
 }
 
 }  // namespace sma

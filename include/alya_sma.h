@@ -185,6 +185,12 @@ int32_t sma_eval_law160(int64_t n, const double* props, double e_mart,
                         const double* d_F, const double* d_tmp,
                         const double* d_sdv_old, double* d_sdv_new, double* d_pk2,
                         int32_t* d_nr_flag, int32_t precision, void* stream);
+/* The same with row-major deformation gradients, F[9g + 3i + j] = F(i,j) (a C
+ * or NumPy (n,3,3) array); pk2 stays column-major. */
+int32_t sma_eval_law160_rowmajor(int64_t n, const double* props, double e_mart,
+                                 const double* d_F, const double* d_tmp,
+                                 const double* d_sdv_old, double* d_sdv_new, double* d_pk2,
+                                 int32_t* d_nr_flag, int32_t precision, void* stream);
 
 /* The same plugin with flagt = 1 (FP64): also the algorithmic tangent
  * d_dds (81n), dds[i + 3j + 9k + 27l + 81g] = gpdds(i,j,k,l,igaus), from
@@ -194,6 +200,10 @@ int32_t sma_eval_law160_tangent(int64_t n, const double* props, double e_mart,
                                 const double* d_F, const double* d_tmp,
                                 const double* d_sdv_old, double* d_sdv_new, double* d_pk2,
                                 double* d_dds, int32_t* d_nr_flag, void* stream);
+int32_t sma_eval_law160_tangent_rowmajor(int64_t n, const double* props, double e_mart,
+                                         const double* d_F, const double* d_tmp,
+                                         const double* d_sdv_old, double* d_sdv_new, double* d_pk2,
+                                         double* d_dds, int32_t* d_nr_flag, void* stream);
 
 /* Element loop that allocates nothing.  No counterpart in the reference:
  * it exists for callers that cannot allocate device memory themselves
