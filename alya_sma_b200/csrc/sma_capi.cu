@@ -404,19 +404,23 @@ using ElemKernel = void (*)(ElemArgs<T>);
 // one-tile kernels: the narrow instance (tighter register cap, more warps)
 // for blocks of up to ELEM_NARROW_BLOCK threads, the wide one above
 template <typename T, bool ATOMIC, bool MATS>
-ElemKernel<T> elem_kernel_v(bool pipe, int block) {
+ElemKernel<T> elem_kernel_v(bool pipe, bool narrow) {
   if (pipe) return k_element_pipe<T, ATOMIC, MATS>;
-  return block <= ELEM_NARROW_BLOCK ? k_element<T, ATOMIC, MATS, false, true> : k_element<T, ATOMIC, MATS>;
+  return narrow ? k_element<T, ATOMIC, MATS, false, true> : k_element<T, ATOMIC, MATS>;
 }
 
+// A launch of at most WIDE_WARPS warps per SM is resident at once also with
+// the wide instance's registers, and takes it for having no spills: the time
+// of such a launch is one element's latency
+constexpr int WIDE_WARPS = 16;
+
 template <typename T>
-ElemKernel<T> elem_kernel(const sma_ctx* c) {
+ElemKernel<T> elem_kernel(const sma_ctx* c, int nelem) {
   const bool pipe = c->variant == SMA_VARIANT_PIPE;
   const bool atomic = c->scatter != SMA_SCATTER_COLOR;
   const bool mats = c->d_lmate != nullptr;
-  const int b = c->block;
+  const bool narrow = c->block <= ELEM_NARROW_BLOCK && nelem > 4 * WIDE_WARPS * c->nsm;
   if (c->compact) {                                              // one-tile, undamped
-    const bool narrow = b <= ELEM_NARROW_BLOCK;
     if (atomic) return narrow ? k_element<T, true, true, false, true, true> : k_element<T, true, true, false, false, true>;
     return narrow ? k_element<T, false, true, false, true, true> : k_element<T, false, true, false, false, true>;
   }
@@ -424,8 +428,8 @@ ElemKernel<T> elem_kernel(const sma_ctx* c) {
     if (atomic) return mats ? k_element<T, true, true, true> : k_element<T, true, false, true>;
     return mats ? k_element<T, false, true, true> : k_element<T, false, false, true>;
   }
-  if (atomic) return mats ? elem_kernel_v<T, true, true>(pipe, b) : elem_kernel_v<T, true, false>(pipe, b);
-  return mats ? elem_kernel_v<T, false, true>(pipe, b) : elem_kernel_v<T, false, false>(pipe, b);
+  if (atomic) return mats ? elem_kernel_v<T, true, true>(pipe, narrow) : elem_kernel_v<T, true, false>(pipe, narrow);
+  return mats ? elem_kernel_v<T, false, true>(pipe, narrow) : elem_kernel_v<T, false, false>(pipe, narrow);
 }
 
 template <typename T>
@@ -449,6 +453,24 @@ ElemKernel<T> solo_kernel(const sma_ctx* c) {
 // against 14.9 / 18.9, 250 k 78 / 146 us against 52 / 90.
 int solo_min(const sma_ctx* c) { return 128 * c->nsm; }
 
+// a kernel of the step, resident before its predecessor on the stream has
+// finished (programmatic dependent launch; the kernels wait for it before
+// they touch what it wrote)
+template <typename... P, typename... A>
+cudaError_t launch_step(sma_ctx* c, void (*k)(P...), unsigned grid, int block, size_t smem, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, args...);
+}
+
 // one element range [beg, end), by the thread-per-element kernel where the
 // context has it and the range fills the GPU with it, else 8 lanes per element
 template <typename T>
@@ -458,13 +480,15 @@ int32_t launch_range_t(sma_ctx* c, int beg, int end, bool advance, bool stepping
   if (c->solo && c->solo_block && end - beg >= solo_min(c) && !a.has_grav) {
     const int block = c->solo_block;
     a.pf_ahead = (int64_t)c->nsm * solo_min_blocks<T>() * SOLO_BLOCK;      // one resident wave
-    solo_kernel<T>(c)<<<(unsigned)ceil_div(end - beg, block), block, solo_smem_bytes<T>(block), c->stream>>>(a);
+    CU(launch_step(c, solo_kernel<T>(c), (unsigned)ceil_div(end - beg, block) + (a.ts ? 1 : 0), block,
+                   solo_smem_bytes<T>(block), a));
   } else {
     const int64_t ntiles = ceil_div(end - beg, c->block / 8);
-    const unsigned grid = c->variant == SMA_VARIANT_PIPE
-                              ? (unsigned)std::min<int64_t>(ntiles, (int64_t)c->nsm * c->resident)
-                              : (unsigned)ntiles;
-    elem_kernel<T>(c)<<<grid, c->block, elem_smem<T>(c), c->stream>>>(a);
+    const bool pipe = c->variant == SMA_VARIANT_PIPE;
+    const unsigned grid = (unsigned)(pipe ? std::min<int64_t>(ntiles, (int64_t)c->nsm * c->resident) : ntiles) +
+                          (a.ts ? 1 : 0);
+    if (pipe) elem_kernel<T>(c, end - beg)<<<grid, c->block, elem_smem<T>(c), c->stream>>>(a);
+    else CU(launch_step(c, elem_kernel<T>(c, end - beg), grid, c->block, elem_smem<T>(c), a));
   }
   c->launches++;
   CU(cudaGetLastError());
@@ -481,7 +505,7 @@ int32_t init_element_launch_t(sma_ctx* c) {
   const size_t smem256 = elem_smem<T>(c);
   c->block = block;
   const size_t smem = elem_smem<T>(c);
-  const ElemKernel<T> k = elem_kernel<T>(c);
+  const ElemKernel<T> k = elem_kernel<T>(c, c->nelem);
   CU(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                           (int)std::max<size_t>(smem256, 48 * 1024)));
   CU(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c->resident, k, block, smem));
@@ -511,7 +535,7 @@ int32_t launch_sur_range(sma_ctx* c, int beg, int end, bool advance, bool steppi
   if (end <= beg) return SMA_OK;
   ElemArgs<float> a = elem_args<float>(c, beg, end, advance, stepping);
   const sur::SurElemArgs s = sur_args(c);
-  const unsigned grid = (unsigned)((end - 1) / sur::SUR_EPB - beg / sur::SUR_EPB + 1);
+  const unsigned grid = (unsigned)((end - 1) / sur::SUR_EPB - beg / sur::SUR_EPB + 1) + (a.ts ? 1 : 0);
   if (c->compact) sur::k_element_sur<true><<<grid, sur::SUR_BLOCK, 0, c->stream>>>(a, s);
   else sur::k_element_sur<false><<<grid, sur::SUR_BLOCK, 0, c->stream>>>(a, s);
   c->launches++;
@@ -752,23 +776,19 @@ int32_t launch_rayleigh(sma_ctx* c, const double* vel) {
 }
 
 template <int MODE>
-void launch_nodal_mode(sma_ctx* c, unsigned grid, const NodalArgs& a) {
+cudaError_t launch_nodal_mode(sma_ctx* c, unsigned grid, const NodalArgs& a) {
   const bool en = c->energy && MODE >= 1;
-  if (c->scheme == SMA_SCHEME_TW) {
-    if (en) k_nodal<MODE, SCHEME_TW, true><<<grid, 256, 0, c->stream>>>(a);
-    else k_nodal<MODE, SCHEME_TW, false><<<grid, 256, 0, c->stream>>>(a);
-  } else {
-    if (en) k_nodal<MODE, SCHEME_CD, true><<<grid, 256, 0, c->stream>>>(a);
-    else k_nodal<MODE, SCHEME_CD, false><<<grid, 256, 0, c->stream>>>(a);
-  }
+  void (*k)(NodalArgs) = c->scheme == SMA_SCHEME_TW
+                             ? (en ? k_nodal<MODE, SCHEME_TW, true> : k_nodal<MODE, SCHEME_TW, false>)
+                             : (en ? k_nodal<MODE, SCHEME_CD, true> : k_nodal<MODE, SCHEME_CD, false>);
+  return launch_step(c, k, grid, 256, 0, a);
 }
 
 int32_t launch_nodal(sma_ctx* c, int mode) {
   const unsigned grid = (unsigned)ceil_div(c->npoin, 256);
   NodalArgs a = nodal_args(c);
-  if (mode == 0) launch_nodal_mode<0>(c, grid, a);
-  else if (mode == 1) launch_nodal_mode<1>(c, grid, a);
-  else launch_nodal_mode<2>(c, grid, a);
+  CU(mode == 0 ? launch_nodal_mode<0>(c, grid, a)
+               : (mode == 1 ? launch_nodal_mode<1>(c, grid, a) : launch_nodal_mode<2>(c, grid, a)));
   c->launches++;
   CU(cudaGetLastError());
   if (c->energy && mode >= 1) {
@@ -1255,7 +1275,7 @@ int32_t sma_step_prologue(sma_ctx* c) {
   if (!(c->dtime > 0.0)) return fail(SMA_ERR_STATE, "dtime not set");
   CU(cudaSetDevice(c->dev));
   if (c->nwit > 0) CU(cudaMemsetAsync(c->d_wrow, 0, sizeof(int), c->stream));
-  k_advance_time<<<1, 1, 0, c->stream>>>(c->d_ts, c->d_ft);
+  k_advance_time<<<1, 32, 0, c->stream>>>(c->d_ts, c->d_ft);
   c->launches++;
   return launch_nodal(c, 0);
 }
@@ -1290,7 +1310,7 @@ int32_t sma_step_elements_range(sma_ctx* c, int32_t beg, int32_t end, int32_t fi
                                     : launch_range_t<double>(c, beg, end, first != 0, true);
     }
   } else if (first) {
-    k_advance_time<<<1, 1, 0, c->stream>>>(c->d_ts, c->d_ft);
+    k_advance_time<<<1, 32, 0, c->stream>>>(c->d_ts, c->d_ft);
     c->launches++;
     CU(cudaGetLastError());
   }
@@ -1348,7 +1368,7 @@ int32_t sma_explicit_step(sma_ctx* c, int32_t nsteps) {
   int32_t rc;
   if (c->nwit > 0) CU(cudaMemsetAsync(c->d_wrow, 0, sizeof(int), c->stream));
   // prologue: time of step 1 and its predictor from the boundary state
-  k_advance_time<<<1, 1, 0, c->stream>>>(c->d_ts, c->d_ft);
+  k_advance_time<<<1, 32, 0, c->stream>>>(c->d_ts, c->d_ft);
   c->launches++;
   if ((rc = launch_nodal(c, 0))) return rc;
   if (c->timing) {

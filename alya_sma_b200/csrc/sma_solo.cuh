@@ -276,6 +276,7 @@ __device__ __forceinline__ void solo_gather(const ElemArgs<T>& a, int64_t ec, T*
   using V = typename PairOf<T>::type;
   int nid[8];
   solo_nodes(a, ec, nid);
+  pdl_wait();                                                    // displacement, state, residual
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
     const double* s0 = c == 0 ? a.coord : (c == 1 ? a.coord + 2 * a.npad : a.u + a.npad);
@@ -283,8 +284,8 @@ __device__ __forceinline__ void solo_gather(const ElemArgs<T>& a, int64_t ec, T*
     double v0[8], v1[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-      v0[k] = __ldg(s0 + nid[k]);
-      v1[k] = __ldg(s1 + nid[k]);
+      v0[k] = c == 2 ? ldcur(s0 + nid[k]) : __ldg(s0 + nid[k]);
+      v1[k] = c == 0 ? __ldg(s1 + nid[k]) : ldcur(s1 + nid[k]);
     }
     V w[8];
     w[0] = mk2(T(0), T(0));
@@ -363,7 +364,8 @@ __global__ void __launch_bounds__(SOLO_BLOCK, (solo_min_blocks<T>())) k_element_
   const int64_t e = (int64_t)a.beg + (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool valid = e < a.end;
   const int64_t ec = valid ? e : (int64_t)a.end - 1;
-  if (a.ts && blockIdx.x == 0 && threadIdx.x == 0) advance_time(a.ts, a.ft);
+  pdl_launch();
+  if (time_block(a)) return;
 
   // the connectivity of the element one resident wave ahead, into L2
   if (e + a.pf_ahead < a.end) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.lnods + 8 * (e + a.pf_ahead)));

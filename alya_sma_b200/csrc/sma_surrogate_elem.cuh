@@ -107,7 +107,7 @@ __device__ __forceinline__ void sur_stage(float* row, const float* E, const floa
 template <bool CMP>
 __global__ void __launch_bounds__(SUR_BLOCK, 6) k_element_sur(ElemArgs<float> a, SurElemArgs s) {
   __shared__ __align__(16) float elem_sm[SUR_EPB * ElemSmem<float>::PER_ELEM];
-  if (a.ts && blockIdx.x == 0 && threadIdx.x == 0) advance_time(a.ts, a.ft);
+  if (time_block(a)) return;
   const int lane8 = threadIdx.x & 7, le = threadIdx.x >> 3;
   float* nsm = elem_sm + le * ElemSmem<float>::PER_ELEM;
   float* qsm = nsm + ElemSmem<float>::NODE_STRIDE;
