@@ -202,15 +202,15 @@ class ExplicitSolid:
         an optional caller-owned (npoin, 3) float64 output array (e.g. one
         page-locked with host_register, like displ)."""
         d = np.ascontiguousarray(displ, dtype=np.float64).reshape(self.npoin, 3)
-        out = {q: np.zeros((self.npoin, 3)) for q in ("rhsid", "finte", "fexte", "frxid")}
-        if rhsid is not None:
-            if rhsid.dtype != np.float64 or rhsid.shape != (self.npoin, 3) or not rhsid.flags["C_CONTIGUOUS"]:
-                raise ValueError("rhsid must be a C-contiguous float64 (npoin, 3) array")
-            out["rhsid"] = rhsid
-        out["vmass"] = np.zeros(self.npoin)
-        if not want_all:
-            for q in ("finte", "fexte", "frxid", "vmass"):
-                out[q] = None
+        if rhsid is None:
+            rhsid = np.empty((self.npoin, 3))
+        elif rhsid.dtype != np.float64 or rhsid.shape != (self.npoin, 3) or not rhsid.flags["C_CONTIGUOUS"]:
+            raise ValueError("rhsid must be a C-contiguous float64 (npoin, 3) array")
+        # only what is asked for, and nothing filled that the library fills
+        out = {"rhsid": rhsid}
+        for q in ("finte", "fexte", "frxid"):
+            out[q] = np.empty((self.npoin, 3)) if want_all else None
+        out["vmass"] = np.empty(self.npoin) if want_all else None
         _check(lib().sma_assemble(self._ctx, _p(d), float(fext_scale), _p(out["rhsid"]),
                                   _p(out["finte"]), _p(out["fexte"]), _p(out["frxid"]),
                                   _p(out["vmass"])))
@@ -225,9 +225,9 @@ class ExplicitSolid:
         yz xz xy, von Mises 'seqvm' (npoin,), and with gp_sigma the Cauchy
         stress per Gauss point (nelem, 8, 6).  Evaluated at the current
         displacement from the state the last element loop started from."""
-        out = {k: np.zeros((self.npoin, 6)) for k in ("caust", "green", "lepsi")}
-        out["seqvm"] = np.zeros(self.npoin)
-        gp = np.zeros((self.nelem, 8, 6)) if gp_sigma else None
+        out = {k: np.empty((self.npoin, 6)) for k in ("caust", "green", "lepsi")}
+        out["seqvm"] = np.empty(self.npoin)
+        gp = np.empty((self.nelem, 8, 6)) if gp_sigma else None
         _check(lib().sma_postprocess(self._ctx, _p(out["caust"]), _p(out["green"]), _p(out["lepsi"]),
                                      _p(out["seqvm"]), _p(gp)))
         if gp_sigma:
@@ -237,7 +237,7 @@ class ExplicitSolid:
     # -- data ----------------------------------------------------------------
     def get(self, field):
         n = (self.npoin,) if field == "vmass" else (self.npoin, 3)
-        out = np.zeros(n)
+        out = np.empty(n)
         _check(lib().sma_get_nodal(self._ctx, FIELD[field], _p(out)))
         return out
 
@@ -250,7 +250,7 @@ class ExplicitSolid:
     def state(self):
         """svegm in the reference layout: (nelem, 2, 8, 3), slot 0 = ITER_K,
         slot 1 = TIME_N."""
-        out = np.zeros((self.nelem, 2, 8, 3))
+        out = np.empty((self.nelem, 2, 8, 3))
         _check(lib().sma_get_state(self._ctx, _p(out)))
         return out
 
@@ -286,8 +286,8 @@ class ExplicitSolid:
         postprocess(): 'gpgdi' (F) and 'gppio' (P = F S) as (nelem, 8, 3, 3)
         holding Fortran T(i,j) at [..., j, i], 'gpdet' (nelem, 8) and
         'volum' = (reference volume, deformed volume)."""
-        out = {k: np.zeros((self.nelem, 8, 3, 3)) for k in ("gpgdi", "gppio")}
-        out["gpdet"] = np.zeros((self.nelem, 8))
+        out = {k: np.empty((self.nelem, 8, 3, 3)) for k in ("gpgdi", "gppio")}
+        out["gpdet"] = np.empty((self.nelem, 8))
         out["volum"] = np.zeros(2)
         _check(lib().sma_gauss_fields(self._ctx, _p(out["gpgdi"]), _p(out["gppio"]), _p(out["gpdet"]),
                                       _p(out["volum"])))
