@@ -293,9 +293,11 @@ struct sma_ctx {
   double* d_uprev = nullptr;
   double* d_fintp = nullptr;
   double* d_fextp = nullptr;
-  double* d_en = nullptr;                  // [4..8] totals (ALLIE, ALLWK, ALLKE, EENER, steps)
+  double* d_en = nullptr;                  // [4..8] totals (ALLIE, ALLWK, ALLKE, EENER, steps), [15] block ticket
   double* d_epart = nullptr;               // per-block partial sums of the nodal kernel
   double* d_fray = nullptr;                // Rayleigh alpha nodal force (damped runs), SoA
+  cudaStream_t s_side = nullptr;           // its pass beside the element loop (fork, join)
+  cudaEvent_t ev_side[2] = {nullptr, nullptr};
   double* d_nodal = nullptr;               // one block: coord, u, f | vt, v, a (each SoA [3][npad])
   bool l2_window = false;                  // persisting-L2 window set on the stream
   // pipelined sma_assemble (atomic scatter, >= 2 slabs): slab bounds, node
@@ -827,6 +829,11 @@ NodalArgs nodal_args(sma_ctx* c) {
   a.fint_prev = c->d_fintp;
   a.fext_prev = c->d_fextp;
   a.en_step = c->d_epart;
+  a.en_tot = c->d_en ? c->d_en + 4 : nullptr;
+  a.en_hist = c->d_ehist;
+  a.en_row = c->d_erow;
+  a.en_max_rows = c->ehist_max;
+  a.en_ticket = c->d_en ? (unsigned*)(c->d_en + 15) : nullptr;
   a.fray = (c->damp && c->energy) ? c->d_fray : nullptr;
   a.store_v = (c->damp && c->scheme == SMA_SCHEME_CD) ? 1 : 0;
   a.npoin = c->npoin;
@@ -835,12 +842,30 @@ NodalArgs nodal_args(sma_ctx* c) {
 }
 
 // the Rayleigh alpha force alone into d_fray (energy balance, finte)
-int32_t launch_rayleigh(sma_ctx* c, const double* vel) {
-  CU(cudaMemsetAsync(c->d_fray, 0, 3 * (size_t)c->npad * sizeof(double), c->stream));
-  k_rayleigh<<<(unsigned)ceil_div(c->nelem, 128), 128, 0, c->stream>>>(
+int32_t launch_rayleigh(sma_ctx* c, const double* vel, cudaStream_t s) {
+  CU(cudaMemsetAsync(c->d_fray, 0, 3 * (size_t)c->npad * sizeof(double), s));
+  k_rayleigh<<<(unsigned)ceil_div(c->nelem, 128), 128, 0, s>>>(
       c->d_lnods, c->d_coord, vel, c->d_lmate, c->d_mats, c->mat0, c->nelem, c->npad, c->d_fray);
   c->launches++;
   CU(cudaGetLastError());
+  return SMA_OK;
+}
+
+// The same within a step, on the side stream from before the element loop
+// (which does not touch d_fray) to the nodal update: its memory traffic and
+// launches hide behind the element kernel and its last wave.
+// 80 k-element FP64 damped cantilever with the energy balance: @RAY@.
+bool side_rayleigh(const sma_ctx* c) { return c->damp && c->energy; }
+int32_t fork_rayleigh(sma_ctx* c) {
+  CU(cudaEventRecord(c->ev_side[0], c->stream));
+  CU(cudaStreamWaitEvent(c->s_side, c->ev_side[0], 0));
+  const int32_t rc = launch_rayleigh(c, damp_velocity(c, true), c->s_side);
+  if (rc) return rc;
+  CU(cudaEventRecord(c->ev_side[1], c->s_side));
+  return SMA_OK;
+}
+int32_t join_rayleigh(sma_ctx* c) {
+  CU(cudaStreamWaitEvent(c->stream, c->ev_side[1], 0));
   return SMA_OK;
 }
 
@@ -850,6 +875,10 @@ cudaError_t launch_nodal_mode(sma_ctx* c, unsigned grid, const NodalArgs& a) {
   void (*k)(NodalArgs) = c->scheme == SMA_SCHEME_TW
                              ? (en ? k_nodal<MODE, SCHEME_TW, true> : k_nodal<MODE, SCHEME_TW, false>)
                              : (en ? k_nodal<MODE, SCHEME_CD, true> : k_nodal<MODE, SCHEME_CD, false>);
+  if (side_rayleigh(c)) {                                         // joins two streams: an ordinary launch
+    k<<<grid, 256, 0, c->stream>>>(a);
+    return cudaGetLastError();
+  }
   return launch_step(c, k, grid, 256, 0, a);
 }
 
@@ -860,13 +889,6 @@ int32_t launch_nodal(sma_ctx* c, int mode) {
                : (mode == 1 ? launch_nodal_mode<1>(c, grid, a) : launch_nodal_mode<2>(c, grid, a)));
   c->launches++;
   CU(cudaGetLastError());
-  if (c->energy && mode >= 1) {
-    k_energy_finalize<<<1, 256, 0, c->stream>>>(c->d_epart, (int)ceil_div(c->npoin, 256), c->d_en + 4,
-                                                 c->d_ehist, c->d_erow,
-                                               c->ehist_max);
-    c->launches++;
-    CU(cudaGetLastError());
-  }
   return SMA_OK;
 }
 
@@ -881,12 +903,13 @@ int32_t launch_witness(sma_ctx* c) {
 
 // one interior step: element loop (advancing time) + fused nodal update
 int32_t issue_step(sma_ctx* c, int nodal_mode) {
-  int32_t rc = launch_elements(c, true);
-  if (rc) return rc;
+  int32_t rc;
+  if (side_rayleigh(c) && (rc = fork_rayleigh(c))) return rc;
+  if ((rc = launch_elements(c, true))) return rc;
   c->cur ^= 1;   // the state written by this step is TIME_N of the next
   // u holds u_k until the nodal kernel predicts u_{k+1}
   if ((rc = launch_witness(c))) return rc;
-  if (c->damp && c->energy && (rc = launch_rayleigh(c, damp_velocity(c, true)))) return rc;
+  if (side_rayleigh(c) && (rc = join_rayleigh(c))) return rc;
   return launch_nodal(c, nodal_mode);
 }
 
@@ -906,11 +929,12 @@ int32_t next_event(sma_ctx* c, int* idx) {
 int32_t issue_step_timed(sma_ctx* c, int nodal_mode) {
   int e0, e1, e2, rc;
   if ((rc = next_event(c, &e0))) return rc;
+  if (side_rayleigh(c) && (rc = fork_rayleigh(c))) return rc;
   if ((rc = launch_elements(c, true))) return rc;
   c->cur ^= 1;
   if ((rc = next_event(c, &e1))) return rc;
   if ((rc = launch_witness(c))) return rc;
-  if (c->damp && c->energy && (rc = launch_rayleigh(c, damp_velocity(c, true)))) return rc;
+  if (side_rayleigh(c) && (rc = join_rayleigh(c))) return rc;
   if ((rc = launch_nodal(c, nodal_mode))) return rc;
   if ((rc = next_event(c, &e2))) return rc;
   c->evmarks.push_back({0, {e0, e1}});
@@ -972,8 +996,7 @@ int64_t kernels_per_step(const sma_ctx* c) {
     for (size_t r = 0; r < c->plan_end.size(); ++r)
       elem += c->plan_end[r] > (r ? c->plan_end[r - 1] : 0);
   }
-  return elem + 1 + (c->sur ? 1 : 0) + (c->nwit > 0 ? 1 : 0) + (c->energy ? 1 : 0) +
-         (c->energy && c->damp ? 1 : 0);
+  return elem + 1 + (c->sur ? 1 : 0) + (c->nwit > 0 ? 1 : 0) + (c->energy && c->damp ? 1 : 0);
 }
 
 template <typename T>
@@ -1012,6 +1035,9 @@ int32_t sma_ctx_destroy(sma_ctx* c) {
     if (b) cudaFree(b);
   for (cudaEvent_t e : c->pl_ev) cudaEventDestroy(e);
   if (c->h_bounce) cudaFreeHost(c->h_bounce);
+  for (cudaEvent_t e : c->ev_side)
+    if (e) cudaEventDestroy(e);
+  if (c->s_side) cudaStreamDestroy(c->s_side);
   if (c->s_h2d) cudaStreamDestroy(c->s_h2d);
   if (c->s_d2h) cudaStreamDestroy(c->s_d2h);
   if (c->stream) cudaStreamDestroy(c->stream);
@@ -1255,6 +1281,8 @@ int32_t sma_ctx_create(const sma_mesh_desc* mesh, const sma_material_desc* mat,
   if (c->damp) {
     TRY(dalloc(&c->d_fray, nb));
     TRYCU(cudaMemset(c->d_fray, 0, nb));
+    TRYCU(cudaStreamCreateWithFlags(&c->s_side, cudaStreamNonBlocking));
+    for (cudaEvent_t& e : c->ev_side) TRYCU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   }
   TRY(dalloc(&c->d_stage, 3 * (size_t)c->npoin * sizeof(double)));
   TRY(dalloc(&c->d_stage2, 3 * (size_t)c->npoin * sizeof(double)));
@@ -1362,7 +1390,7 @@ int32_t sma_step_elements(sma_ctx* c) {
   if (rc) return rc;
   c->cur ^= 1;
   if ((rc = launch_witness(c))) return rc;
-  if (c->damp && c->energy && (rc = launch_rayleigh(c, damp_velocity(c, true)))) return rc;
+  if (c->damp && c->energy && (rc = launch_rayleigh(c, damp_velocity(c, true), c->stream))) return rc;
   return SMA_OK;
 }
 
@@ -1394,7 +1422,7 @@ int32_t sma_step_elements_range(sma_ctx* c, int32_t beg, int32_t end, int32_t fi
   if (last) {
     c->cur ^= 1;
     if ((rc = launch_witness(c))) return rc;
-    if (c->damp && c->energy && (rc = launch_rayleigh(c, damp_velocity(c, true)))) return rc;
+    if (c->damp && c->energy && (rc = launch_rayleigh(c, damp_velocity(c, true), c->stream))) return rc;
   }
   return SMA_OK;
 }
@@ -1513,7 +1541,7 @@ int32_t sma_assemble(sma_ctx* c, const double* displ, double fext_scale, double*
   // with damping, finte leaves the Rayleigh force out (it is in rhsid only)
   const double* fray = nullptr;
   if (c->damp && finte) {
-    if ((rc = launch_rayleigh(c, damp_velocity(c, false)))) return rc;
+    if ((rc = launch_rayleigh(c, damp_velocity(c, false), c->stream))) return rc;
     fray = c->d_fray;
   }
   for (int q = piped ? 1 : 0; q < 4; ++q) {

@@ -1001,12 +1001,56 @@ struct NodalArgs {
   double* fint_prev;
   double* fext_prev;
   double* en_step;
+  double* en_tot;         // totals (energy_finalize), history and its row counter
+  double* en_hist;
+  int* en_row;
+  int en_max_rows;
+  unsigned* en_ticket;    // blocks done; 0 between launches
   const double* fray;     // Rayleigh alpha nodal force of the step (kept out of fint), or null
   int store_v;            // MODE 1 also stores the step-boundary velocity (damped CD runs)
   int64_t npoin, npad;
 };
 
 constexpr int SCHEME_CD = 0, SCHEME_TW = 1;
+
+// Energy totals after a step (mod_sld_energy.f90:130-157): increments are
+// taken in absolute value, halved except on the first step; one history row
+// (ALLIE, ALLWK, ALLKE, ETOTA, EENER) per step.  By the nodal kernel's last
+// block (256 threads): the blocks' partials summed in a fixed order (strided
+// per thread, then a tree), so the balance is bitwise reproducible.  In a
+// kernel of its own it cost the step @FIN@.
+__device__ __forceinline__ void energy_finalize(const double* part, int nblocks, double* en_tot, double* hist, int* row,
+                                                int max_rows) {
+  __shared__ double red[256][4];
+  double s[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int b = threadIdx.x; b < nblocks; b += 256)
+    for (int q = 0; q < 4; ++q) s[q] += __ldcg(part + 4 * (int64_t)b + q);   // other blocks' writes: from L2
+  for (int q = 0; q < 4; ++q) red[threadIdx.x][q] = s[q];
+  __syncthreads();
+  for (int w = 128; w > 0; w >>= 1) {
+    if ((int)threadIdx.x < w)
+      for (int q = 0; q < 4; ++q) red[threadIdx.x][q] += red[threadIdx.x + w][q];
+    __syncthreads();
+  }
+  if (threadIdx.x != 0) return;
+  const bool first = en_tot[4] == 0.0;
+  const double w = first ? 1.0 : 0.5;
+  en_tot[0] += w * fabs(red[0][0]);
+  en_tot[1] += w * fabs(red[0][1]);
+  en_tot[2] = 0.5 * red[0][2];
+  en_tot[3] = fabs(red[0][3]);
+  en_tot[4] += 1.0;
+  const int r = *row;
+  if (hist && r < max_rows) {
+    double* h = hist + 5 * (int64_t)r;
+    h[0] = en_tot[0];
+    h[1] = en_tot[1];
+    h[2] = en_tot[2];
+    h[3] = en_tot[0] + en_tot[2] - en_tot[1];
+    h[4] = en_tot[3];
+  }
+  *row = r + 1;
+}
 
 // MODE 0: predictor of step k+1 from the step-boundary state
 // MODE 1: corrector of step k fused with the predictor of step k+1
@@ -1107,51 +1151,22 @@ __global__ void __launch_bounds__(256) k_nodal(NodalArgs a) {
       double s = 0.0;
       for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += wsum[w][threadIdx.x];
       a.en_step[4 * (int64_t)blockIdx.x + threadIdx.x] = s;
+      __threadfence();                                           // before this block's ticket
+    }
+    __shared__ bool last;
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(a.en_ticket, 1u) == gridDim.x - 1;
+    __syncthreads();
+    if (last) {                                                  // every block's partial is out
+      __threadfence();
+      energy_finalize(a.en_step, (int)gridDim.x, a.en_tot, a.en_hist, a.en_row, a.en_max_rows);
+      if (threadIdx.x == 0) *a.en_ticket = 0u;
     }
   }
   if (MODE != 2 && blockIdx.x == 0 && threadIdx.x == 0) {
     a.ts->cutim = a.ts->nx_cutim;
     a.ts->load = a.ts->nx_load;
   }
-}
-
-// energy totals after a step (mod_sld_energy.f90:130-157): increments are
-// taken in absolute value, halved except on the first step; one history row
-// (ALLIE, ALLWK, ALLKE, ETOTA, EENER) per step
-// one block of 256 threads: the nodal kernel's per-block partials summed in
-// a fixed order (strided per thread, then a tree), then the totals
-__global__ void __launch_bounds__(256) k_energy_finalize(const double* part, int nblocks,
-                                                         double* en_tot, double* hist, int* row,
-                                                         int max_rows) {
-  __shared__ double red[256][4];
-  double s[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int b = threadIdx.x; b < nblocks; b += 256)
-    for (int q = 0; q < 4; ++q) s[q] += part[4 * (int64_t)b + q];
-  for (int q = 0; q < 4; ++q) red[threadIdx.x][q] = s[q];
-  __syncthreads();
-  for (int w = 128; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w)
-      for (int q = 0; q < 4; ++q) red[threadIdx.x][q] += red[threadIdx.x + w][q];
-    __syncthreads();
-  }
-  if (threadIdx.x != 0) return;
-  const bool first = en_tot[4] == 0.0;
-  const double w = first ? 1.0 : 0.5;
-  en_tot[0] += w * fabs(red[0][0]);
-  en_tot[1] += w * fabs(red[0][1]);
-  en_tot[2] = 0.5 * red[0][2];
-  en_tot[3] = fabs(red[0][3]);
-  en_tot[4] += 1.0;
-  const int r = *row;
-  if (hist && r < max_rows) {
-    double* h = hist + 5 * (int64_t)r;
-    h[0] = en_tot[0];
-    h[1] = en_tot[1];
-    h[2] = en_tot[2];
-    h[3] = en_tot[0] + en_tot[2] - en_tot[1];
-    h[4] = en_tot[3];
-  }
-  *row = r + 1;
 }
 
 // witness: after the element loop of a step, record displacement (ids in
