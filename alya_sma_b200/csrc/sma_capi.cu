@@ -545,10 +545,10 @@ cudaError_t launch_step(sma_ctx* c, void (*k)(P...), unsigned grid, int block, s
 // one element range [beg, end), by the thread-per-element kernel where the
 // context has it and the range fills the GPU with it, else 8 lanes per element
 template <typename T>
-int32_t launch_range_t(sma_ctx* c, int beg, int end, bool advance, bool stepping) {
+int32_t launch_range_t(sma_ctx* c, int beg, int end, bool advance, bool stepping, bool beside = false) {
   if (end <= beg) return SMA_OK;
   ElemArgs<T> a = elem_args<T>(c, beg, end, advance, stepping);
-  if (c->solo && c->solo_block && end - beg >= solo_min(c) && !a.has_grav) {
+  if (c->solo && c->solo_block && end - beg >= solo_min(c) && !a.has_grav && (!c->damp || beside)) {
     const int block = c->solo_block;
     a.pf_ahead = (int64_t)c->nsm * solo_min_blocks<T>() * SOLO_BLOCK;      // one resident wave
     CU(launch_step(c, solo_kernel<T>(c), (unsigned)ceil_div(end - beg, block) + (a.ts ? 1 : 0), block,
@@ -678,8 +678,9 @@ int32_t launch_plan_t(sma_ctx* c, bool advance) {
   return SMA_OK;
 }
 
+// beside: the damping force is added by the side pass
 template <typename T>
-int32_t launch_elements_t(sma_ctx* c, bool advance) {
+int32_t launch_elements_t(sma_ctx* c, bool advance, bool beside) {
   const int nrange = (int)c->cptr.size() - 1;
   if (c->resident == 0) return fail(SMA_ERR_STATE, "element launch not initialised");
   if constexpr (sizeof(T) == 4) {
@@ -695,15 +696,15 @@ int32_t launch_elements_t(sma_ctx* c, bool advance) {
   }
   c->last_in = c->cur;
   for (int r = 0; r < nrange; ++r) {
-    const int32_t rc = launch_range_t<T>(c, c->cptr[r], c->cptr[r + 1], advance && r == 0, advance);
+    const int32_t rc = launch_range_t<T>(c, c->cptr[r], c->cptr[r + 1], advance && r == 0, advance, beside);
     if (rc) return rc;
   }
   return SMA_OK;
 }
 
-int32_t launch_elements(sma_ctx* c, bool advance) {
-  return c->prec == SMA_PREC_FP32 ? launch_elements_t<float>(c, advance)
-                                  : launch_elements_t<double>(c, advance);
+int32_t launch_elements(sma_ctx* c, bool advance, bool beside = false) {
+  return c->prec == SMA_PREC_FP32 ? launch_elements_t<float>(c, advance, beside)
+                                  : launch_elements_t<double>(c, advance, beside);
 }
 
 // one element range [beg, end) of an atomic-scatter context outside a step
@@ -842,10 +843,11 @@ NodalArgs nodal_args(sma_ctx* c) {
 }
 
 // the Rayleigh alpha force alone into d_fray (energy balance, finte)
-int32_t launch_rayleigh(sma_ctx* c, const double* vel, cudaStream_t s) {
-  CU(cudaMemsetAsync(c->d_fray, 0, 3 * (size_t)c->npad * sizeof(double), s));
+int32_t launch_rayleigh(sma_ctx* c, const double* vel, cudaStream_t s, bool force = true, double* rhs = nullptr) {
+  if (force) CU(cudaMemsetAsync(c->d_fray, 0, 3 * (size_t)c->npad * sizeof(double), s));
   k_rayleigh<<<(unsigned)ceil_div(c->nelem, 128), 128, 0, s>>>(
-      c->d_lnods, c->d_coord, vel, c->d_lmate, c->d_mats, c->mat0, c->nelem, c->npad, c->d_fray);
+      c->d_lnods, c->d_coord, vel, c->d_lmate, c->d_mats, c->mat0, c->nelem, c->npad, force ? c->d_fray : nullptr,
+      rhs);
   c->launches++;
   CU(cudaGetLastError());
   return SMA_OK;
@@ -854,12 +856,21 @@ int32_t launch_rayleigh(sma_ctx* c, const double* vel, cudaStream_t s) {
 // The same within a step, on the side stream from before the element loop
 // (which does not touch d_fray) to the nodal update: its memory traffic and
 // launches hide behind the element kernel and its last wave.
-// 80 k-element FP64 damped cantilever with the energy balance: @RAY@.
-bool side_rayleigh(const sma_ctx* c) { return c->damp && c->energy; }
+// 80 k-element FP64 damped cantilever with the energy balance: 61.6 -> 60.3 us
+// per step.
+// Where the context has the thread-per-element kernel, which has no damping,
+// the side pass also puts the force into the residual (per step, 8 damped
+// lanes per element against one thread and the side pass: 80 k elements FP64
+// 48.0 / 38.8 us, with the energy balance 60.2 / 46.4, FP32 30.9 / 26.9; 250 k
+// cylinder FP32 121 / 110; below two warps per scheduler the second launch
+// costs more than it gives: 25.6 k FP32 15.4 / 17.0).
+bool damp_beside(const sma_ctx* c) { return c->damp && c->solo && c->plan_end.empty(); }
+bool side_rayleigh(const sma_ctx* c) { return c->damp && (c->energy || damp_beside(c)); }
 int32_t fork_rayleigh(sma_ctx* c) {
   CU(cudaEventRecord(c->ev_side[0], c->stream));
   CU(cudaStreamWaitEvent(c->s_side, c->ev_side[0], 0));
-  const int32_t rc = launch_rayleigh(c, damp_velocity(c, true), c->s_side);
+  const int32_t rc =
+      launch_rayleigh(c, damp_velocity(c, true), c->s_side, c->energy, damp_beside(c) ? c->d_f : nullptr);
   if (rc) return rc;
   CU(cudaEventRecord(c->ev_side[1], c->s_side));
   return SMA_OK;
@@ -905,7 +916,7 @@ int32_t launch_witness(sma_ctx* c) {
 int32_t issue_step(sma_ctx* c, int nodal_mode) {
   int32_t rc;
   if (side_rayleigh(c) && (rc = fork_rayleigh(c))) return rc;
-  if ((rc = launch_elements(c, true))) return rc;
+  if ((rc = launch_elements(c, true, damp_beside(c)))) return rc;
   c->cur ^= 1;   // the state written by this step is TIME_N of the next
   // u holds u_k until the nodal kernel predicts u_{k+1}
   if ((rc = launch_witness(c))) return rc;
@@ -930,7 +941,7 @@ int32_t issue_step_timed(sma_ctx* c, int nodal_mode) {
   int e0, e1, e2, rc;
   if ((rc = next_event(c, &e0))) return rc;
   if (side_rayleigh(c) && (rc = fork_rayleigh(c))) return rc;
-  if ((rc = launch_elements(c, true))) return rc;
+  if ((rc = launch_elements(c, true, damp_beside(c)))) return rc;
   c->cur ^= 1;
   if ((rc = next_event(c, &e1))) return rc;
   if ((rc = launch_witness(c))) return rc;
@@ -996,7 +1007,7 @@ int64_t kernels_per_step(const sma_ctx* c) {
     for (size_t r = 0; r < c->plan_end.size(); ++r)
       elem += c->plan_end[r] > (r ? c->plan_end[r - 1] : 0);
   }
-  return elem + 1 + (c->sur ? 1 : 0) + (c->nwit > 0 ? 1 : 0) + (c->energy && c->damp ? 1 : 0);
+  return elem + 1 + (c->sur ? 1 : 0) + (c->nwit > 0 ? 1 : 0) + (side_rayleigh(c) ? 1 : 0);
 }
 
 template <typename T>
@@ -1201,8 +1212,8 @@ int32_t sma_ctx_create(const sma_mesh_desc* mesh, const sma_material_desc* mat,
   TRY(dalloc(&c->d_mats, mats.size() * sizeof(MatC)));
   TRYCU(cudaMemcpy(c->d_mats, mats.data(), mats.size() * sizeof(MatC), cudaMemcpyHostToDevice));
   c->mat0 = mats[0];
-  c->solo = run->variant == SMA_VARIANT_AUTO && c->scatter == SMA_SCATTER_ATOMIC && !c->damp &&
-            run->block <= SOLO_BLOCK && c->nelem >= solo_min(c);
+  c->solo = run->variant == SMA_VARIANT_AUTO && c->scatter == SMA_SCATTER_ATOMIC &&
+            run->block <= SOLO_BLOCK && c->nelem >= (c->damp ? 2 : 1) * solo_min(c);
   if (c->solo) {
     if (run->block) c->solo_block = run->block;
     c->sst = 8 * (ceil_div(c->nelem, 32) * 32);                 // whole tiles: 3 sst values

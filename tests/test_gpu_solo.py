@@ -150,3 +150,41 @@ def test_surrogate_and_postprocessing_read_the_tiled_state():
     (p0, r0), (p1, r1) = out
     assert np.linalg.norm(p0 - p1) <= 1e-4 * np.linalg.norm(p0)
     assert np.abs(r0 - r1).max() <= 1e-6 * np.abs(r0).max()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("scheme,energy", [("cd", True), ("cd", False), ("tw", True)])
+def test_damped_steps_equal_the_8_lane_kernel(precision, scheme, energy):
+    """39,884 elements, above two warps per scheduler: the damping force comes
+    from the pass beside the element loop."""
+    coord, lnods = P.structured_box(59, 26, 26, 59.0, 26.0, 26.0, 0.05, 5)
+    base = _mesh("one")
+    npo = len(coord)
+    fixno = np.zeros((npo, 3), np.int32)
+    fixno[P.face_nodes(coord, 0, 0.0)] = 1
+    prob = dataclasses.replace(base, coord=coord, lnods=lnods, fixno=fixno, bcfun=np.full(npo, -1, np.int32),
+                               fext=P.face_load(coord, lnods, 0, 59.0, (1.0, 0.0, 0.0)),
+                               dampi=np.array([[2.0e5, 0.0]]))
+    u = P.prestrain(prob, 0.01)
+    v = 1.0e3 * np.random.default_rng(1).normal(size=u.shape)
+    a = sma.ExplicitSolid(prob, precision=precision, scheme=scheme)
+    b = sma.ExplicitSolid(prob, precision=precision, scheme=scheme, variant="plain")
+    for s in (a, b):
+        s.set("displ", u)
+        s.set("veloc", v)
+        if energy:
+            s.set_energy(True, 32)
+        s.step(3)
+        s.step(20)                                          # eager steps and graphs
+    tol = 1e-10 if precision == "fp64" else 1e-4
+    for f in ("displ", "veloc"):
+        x, y = a.get(f), b.get(f)
+        assert np.linalg.norm(x - y) <= tol * np.linalg.norm(y), f
+    ra, rb = (s.assemble(u, fext_scale=0.5) for s in (a, b))
+    for k in ("rhsid", "finte", "frxid"):
+        assert np.linalg.norm(ra[k] - rb[k]) <= tol * np.linalg.norm(rb[k]), k
+    if energy:
+        (ta, ha), (tb, hb) = a.energy(), b.energy()
+        assert len(ha) == len(hb) == 23
+        for k in ("allie", "allke", "eener"):
+            assert abs(ta[k] - tb[k]) <= 10 * tol * abs(tb[k]), k
