@@ -919,8 +919,8 @@ int32_t issue_step(sma_ctx* c, int nodal_mode) {
   if ((rc = launch_elements(c, true, damp_beside(c)))) return rc;
   c->cur ^= 1;   // the state written by this step is TIME_N of the next
   // u holds u_k until the nodal kernel predicts u_{k+1}
+  if (side_rayleigh(c) && (rc = join_rayleigh(c))) return rc;    // a residual witness records the whole force
   if ((rc = launch_witness(c))) return rc;
-  if (side_rayleigh(c) && (rc = join_rayleigh(c))) return rc;
   return launch_nodal(c, nodal_mode);
 }
 
@@ -944,8 +944,8 @@ int32_t issue_step_timed(sma_ctx* c, int nodal_mode) {
   if ((rc = launch_elements(c, true, damp_beside(c)))) return rc;
   c->cur ^= 1;
   if ((rc = next_event(c, &e1))) return rc;
+  if (side_rayleigh(c) && (rc = join_rayleigh(c))) return rc;    // a residual witness records the whole force
   if ((rc = launch_witness(c))) return rc;
-  if (side_rayleigh(c) && (rc = join_rayleigh(c))) return rc;
   if ((rc = launch_nodal(c, nodal_mode))) return rc;
   if ((rc = next_event(c, &e2))) return rc;
   c->evmarks.push_back({0, {e0, e1}});

@@ -152,19 +152,22 @@ def test_surrogate_and_postprocessing_read_the_tiled_state():
     assert np.abs(r0 - r1).max() <= 1e-6 * np.abs(r0).max()
 
 
-@pytest.mark.parametrize("precision", ["fp64", "fp32"])
-@pytest.mark.parametrize("scheme,energy", [("cd", True), ("cd", False), ("tw", True)])
-def test_damped_steps_equal_the_8_lane_kernel(precision, scheme, energy):
+def _damped_mesh():
     """39,884 elements, above two warps per scheduler: the damping force comes
     from the pass beside the element loop."""
     coord, lnods = P.structured_box(59, 26, 26, 59.0, 26.0, 26.0, 0.05, 5)
-    base = _mesh("one")
     npo = len(coord)
     fixno = np.zeros((npo, 3), np.int32)
     fixno[P.face_nodes(coord, 0, 0.0)] = 1
-    prob = dataclasses.replace(base, coord=coord, lnods=lnods, fixno=fixno, bcfun=np.full(npo, -1, np.int32),
+    return dataclasses.replace(_mesh("one"), coord=coord, lnods=lnods, fixno=fixno, bcfun=np.full(npo, -1, np.int32),
                                fext=P.face_load(coord, lnods, 0, 59.0, (1.0, 0.0, 0.0)),
                                dampi=np.array([[2.0e5, 0.0]]))
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("scheme,energy", [("cd", True), ("cd", False), ("tw", True)])
+def test_damped_steps_equal_the_8_lane_kernel(precision, scheme, energy):
+    prob = _damped_mesh()
     u = P.prestrain(prob, 0.01)
     v = 1.0e3 * np.random.default_rng(1).normal(size=u.shape)
     a = sma.ExplicitSolid(prob, precision=precision, scheme=scheme)
@@ -188,3 +191,41 @@ def test_damped_steps_equal_the_8_lane_kernel(precision, scheme, energy):
         assert len(ha) == len(hb) == 23
         for k in ("allie", "allke", "eener"):
             assert abs(ta[k] - tb[k]) <= 10 * tol * abs(tb[k]), k
+
+
+@pytest.mark.parametrize("timed", [False, True])
+@pytest.mark.parametrize("scheme,energy", [("cd", False), ("cd", True), ("tw", False)])
+def test_residual_witnesses_hold_the_damping_force(scheme, energy, timed):
+    """Residual witnesses of a damped run record the whole residual of every
+    step, eager, captured or timed, with the force of the pass beside the
+    element loop in it."""
+    prob = _damped_mesh()
+    u = P.prestrain(prob, 0.01)
+    v = 1.0e3 * np.random.default_rng(1).normal(size=u.shape)
+    rng = np.random.default_rng(2)
+    free = 3 * prob.npoin + rng.choice(3 * prob.npoin, 2000, replace=False)
+    root = P.face_nodes(prob.coord, 0, 0.0)
+    wit = np.concatenate([free, 3 * prob.npoin + 3 * root, 3 * rng.choice(prob.npoin, 50, replace=False)])
+    h = []
+    for variant, damped in (("auto", True), ("plain", True), ("plain", False)):
+        s = sma.ExplicitSolid(prob if damped else dataclasses.replace(prob, dampi=None), precision="fp64",
+                              scheme=scheme, variant=variant)
+        s.set("displ", u)
+        s.set("veloc", v)
+        s.set_energy(energy, 32)
+        s.set_witness(wit, 32)
+        s.set_timing(timed)
+        rows = []
+        for n in (3, 20):                                   # eager steps, then graphs; a call's rows
+            s.step(n)
+            rows.append(s.witness())
+        h.append(np.concatenate(rows))
+    a, b, und = h
+    assert a.shape == b.shape == (23, len(wit))
+    nf = len(wit) - 50                                      # residuals, then displacements
+    for x, y in zip(a, b):
+        scale = np.linalg.norm(y[:nf])
+        assert np.linalg.norm(x[:nf] - y[:nf]) <= 1e-9 * scale
+        assert np.linalg.norm(x[nf:] - y[nf:]) <= 1e-10 * np.linalg.norm(y[nf:])
+    # the damping force is a part of the first residual that a miss would show
+    assert np.linalg.norm(b[0][:nf] - und[0][:nf]) > 1e-3 * np.linalg.norm(b[0][:nf])
