@@ -249,7 +249,7 @@ struct sma_ctx {
   MatC* d_mats = nullptr;
   MatC mat0;                               // material 0, passed by value when nmate == 1
   void* d_matx = nullptr;                  // compact per-element records (T [nelem][MATX]) or null
-  bool compact = false;                    // element kernel reads d_matx instead of d_mats
+  bool compact = false;                    // the element kernels read them instead of d_mats
   bool many_mats = false;                  // a material per few elements (COMPACT_MAX_SHARING)
   // learned surrogate (FP32 form): weight image, statistics, eps_tr ping-pong
   // per-range element blocks (sma_set_launch_plan): plan_end[r] ends range r
@@ -607,7 +607,7 @@ int32_t launch_sur_range(sma_ctx* c, int beg, int end, bool advance, bool steppi
   ElemArgs<float> a = elem_args<float>(c, beg, end, advance, stepping);
   const sur::SurElemArgs s = sur_args(c);
   const unsigned grid = (unsigned)((end - 1) / sur::SUR_EPB - beg / sur::SUR_EPB + 1) + (a.ts ? 1 : 0);
-  if (c->compact) sur::k_element_sur<true><<<grid, sur::SUR_BLOCK, 0, c->stream>>>(a, s);
+  if (c->d_matx) sur::k_element_sur<true><<<grid, sur::SUR_BLOCK, 0, c->stream>>>(a, s);
   else sur::k_element_sur<false><<<grid, sur::SUR_BLOCK, 0, c->stream>>>(a, s);
   c->launches++;
   CU(cudaGetLastError());
@@ -649,7 +649,7 @@ int32_t sur_init_residuals(sma_ctx* c) {
   const int64_t ntiles = ceil_div(c->nelem, sur::SUR_EPB);
   for (int cls = 0; cls < c->sur_period && cls < ntiles; ++cls) {
     const unsigned grid = (unsigned)ceil_div(ntiles - cls, c->sur_period);
-    if (c->compact) sur::k_sur_stage<true><<<grid, sur::SUR_BLOCK, 0, c->stream>>>(a, sa, cls);
+    if (c->d_matx) sur::k_sur_stage<true><<<grid, sur::SUR_BLOCK, 0, c->stream>>>(a, sa, cls);
     else sur::k_sur_stage<false><<<grid, sur::SUR_BLOCK, 0, c->stream>>>(a, sa, cls);
     c->launches++;
     CU(cudaGetLastError());
@@ -1227,8 +1227,8 @@ int32_t sma_ctx_create(const sma_mesh_desc* mesh, const sma_material_desc* mat,
   // materials, a table the caches hold) +16 % FP32 with 8 lanes per element,
   // so a few materials keep the table there.  One thread per element reads a
   // record once for 8 Gauss points: 24 specimens 82 -> 63 us FP32, 121 -> 107
-  // us FP64, so it always takes records.  The undamped kernels read them;
-  // SMA_VARIANT_TABLE keeps the table.
+  // us FP64, so it takes records for a few materials too.  The undamped
+  // kernels read them; SMA_VARIANT_TABLE keeps the table.
   c->many_mats = (int64_t)c->nmate * COMPACT_MAX_SHARING >= c->nelem;
   if (c->d_lmate && (c->solo || c->many_mats) && c->variant == SMA_VARIANT_PLAIN && !c->damp &&
       run->variant != SMA_VARIANT_TABLE) {
@@ -1251,22 +1251,37 @@ int32_t sma_ctx_create(const sma_mesh_desc* mesh, const sma_material_desc* mat,
         r[MX_RF_SA] = m.Rf_SA;
         r[MX_TEMP] = mat->tempe ? mat->tempe[c->perm[e]] : 0.0;
       }
+      bool exact = true;
       if (c->prec == SMA_PREC_FP32) {
-        // offsets from material 0 (temperature: from the first element's)
+        // offsets from material 0 (temperature: from the first element's),
+        // where they give every value back to 2^-25 of it, half an FP32
+        // rounding at worst (offsets up to half the value always do), and
+        // every temperature to 2^-24 of the largest.  Dissimilar materials (an
+        // elastic region with its thresholds out of reach beside NiTi: 6.7 %
+        // off in a threshold) read the table.
         c->mat0.T0 = rec[MX_TEMP];
+        double tmax = 0.0;
+        for (size_t q = MX_TEMP; q < rec.size(); q += MATX) tmax = std::max(tmax, std::fabs(rec[q]));
         const double base[MATX] = {c->mat0.iEA, c->mat0.iEM, c->mat0.eL, c->mat0.Rs_AS, c->mat0.Rf_AS,
                                    c->mat0.Rs_SA, c->mat0.Rf_SA, c->mat0.T0};
         std::vector<float> rf(rec.size());
-        for (size_t q = 0; q < rec.size(); ++q) rf[q] = (float)(rec[q] - base[q % MATX]);
-        TRY(dalloc(&c->d_matx, rf.size() * sizeof(float)));
-        TRYCU(cudaMemcpy(c->d_matx, rf.data(), rf.size() * sizeof(float), cudaMemcpyHostToDevice));
+        for (size_t q = 0; q < rec.size(); ++q) {
+          const double b = base[q % MATX], v = rec[q];
+          rf[q] = (float)(v - b);
+          exact = exact && std::fabs(b + (double)rf[q] - v) <=
+                               (q % MATX == MX_TEMP ? 0x1p-24 * tmax : 0x1p-25 * std::fabs(v));
+        }
+        if (exact || c->many_mats) {                             // the surrogate reads them in any case
+          TRY(dalloc(&c->d_matx, rf.size() * sizeof(float)));
+          TRYCU(cudaMemcpy(c->d_matx, rf.data(), rf.size() * sizeof(float), cudaMemcpyHostToDevice));
+        }
       } else {
         TRY(dalloc(&c->d_matx, rec.size() * sizeof(double)));
         TRYCU(cudaMemcpy(c->d_matx, rec.data(), rec.size() * sizeof(double), cudaMemcpyHostToDevice));
       }
-      c->compact = true;
+      c->compact = exact;
       // no block barrier: one-warp blocks, as with one material
-      if (!run->block) c->block = 32;
+      if (exact && !run->block) c->block = 32;
     }
   }
 
@@ -2292,7 +2307,7 @@ extern "C" int32_t sma_set_surrogate(sma_ctx* c, const float* params, const sma_
   if (c->prec != SMA_PREC_FP32) return fail(SMA_ERR_ARG, "the surrogate runs in the FP32 precision form");
   if (c->scatter != SMA_SCATTER_ATOMIC) return fail(SMA_ERR_ARG, "the surrogate element loop scatters by atomics");
   if (c->damp) return fail(SMA_ERR_ARG, "the surrogate element loop has no Rayleigh damping");
-  if (c->d_lmate && !(c->compact && c->many_mats))
+  if (c->d_lmate && !(c->d_matx && c->many_mats))
     return fail(SMA_ERR_ARG, "per-element materials need compact records for the surrogate");
   if (!(gate > 0.0) || !(xs_tol >= 0.0) || !(f_margin >= 0.0) || period < 1)
     return fail(SMA_ERR_ARG, "gate > 0, xs_tol >= 0, f_margin >= 0, period >= 1");

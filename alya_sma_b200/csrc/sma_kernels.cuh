@@ -188,9 +188,9 @@ __device__ __forceinline__ int64_t state_at(const ElemArgs<T>& a, int64_t e, int
 // enters through the Reuss rule E(xS0) = 1 / ((1 - xS0)/E_A + xS0/E_M),
 // which is E_A when E_M = E_A.  FP64 forms store the values; FP32 forms store
 // their offsets from mat0's (temperature: from mat0.T0) in FP32, 32 bytes
-// per element, whose rounding (relative 6e-8 of an offset of ~10 %) stays
-// an order below FP32 rounding of the values themselves: with the values
-// rounded to FP32 the thresholds and temperature moved the step at which
+// per element, where every offset gives its value back to half an FP32
+// rounding (sma_ctx_create; spreads of ~10 %: an order below it): with the
+// values rounded to FP32 the thresholds and temperature moved the step at which
 // Gauss points start transforming, and the 2.0 M-element cylinder's 300-step
 // FP32 trajectory parted from the FP64 oracle by 2e-5 instead of 2.5e-6.
 enum MatX { MX_IEA = 0, MX_IEM, MX_EL, MX_RS_AS, MX_RF_AS, MX_RS_SA, MX_RF_SA, MX_TEMP, MATX };

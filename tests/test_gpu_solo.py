@@ -229,3 +229,59 @@ def test_residual_witnesses_hold_the_damping_force(scheme, energy, timed):
         assert np.linalg.norm(x[nf:] - y[nf:]) <= 1e-10 * np.linalg.norm(y[nf:])
     # the damping force is a part of the first residual that a miss would show
     assert np.linalg.norm(b[0][:nf] - und[0][:nf]) > 1e-3 * np.linalg.norm(b[0][:nf])
+
+
+def _two_materials(kind):
+    """(18-parameter rows, martensite moduli, temperatures or None) of a mesh
+    of a few materials that share what compact records do not hold."""
+    base = P.nitinol_props(**P.NITI, C_AS=5.0, C_SA=5.0, T_ref=300.0)
+    pr, em, t = np.stack([base, base]), np.array([P.NITI_E_MART, P.NITI_E_MART]), (300.0, 310.0)
+    if kind == "similar":
+        pr[1, [0, 2, 3, 4, 9, 10]] *= 1.08
+    if kind == "elastic":                                   # material 0: thresholds out of reach
+        pr[0, 3:5], pr[0, 9:11] = (1e9, 2e9), (-1e9, -2e9)
+    if kind == "soft":
+        pr[0, 0] = em[0] = 1.0
+    if kind == "celsius":
+        pr[:, [6, 7, 12, 13]] = -26.85
+        t = (10.0, 90.0)
+    return pr, em, t
+
+
+@pytest.mark.parametrize("many", [False, True])
+@pytest.mark.parametrize("kind,records", [("similar", True), ("celsius", True), ("elastic", False), ("soft", False)])
+def test_fp32_records_only_where_they_hold_the_constants(kind, records, many):
+    """A few (or many) materials in the FP32 form: records of offsets from
+    material 0 where those hold every constant, else the FP64 table; the
+    forces agree with the table's either way."""
+    pr, em, t = _two_materials(kind)
+    base = _mesh("one")
+    ne = base.nelem
+    lmate = np.repeat([0, 1], [ne // 3, ne - ne // 3]).astype(np.int32)
+    if many:                                                # the same two, one row per element
+        pr, em, lmate = pr[lmate], em[lmate], np.arange(ne, dtype=np.int32)
+    prob = dataclasses.replace(base, props=pr, e_mart=em, densi=np.full(len(pr), P.NITI_DENSITY), lmate=lmate,
+                               tempe=np.random.default_rng(5).uniform(*t, ne))
+    u = P.prestrain(prob, 0.012)
+    a = sma.ExplicitSolid(prob, precision="fp32")
+    b = sma.ExplicitSolid(prob, precision="fp32", variant="table")
+    d = sma.ExplicitSolid(prob, precision="fp64", variant="table")
+    assert a.launch_info()["compact_records"] == records and not b.launch_info()["compact_records"]
+    ra, rb, rd = (s.assemble(u)["rhsid"] for s in (a, b, d))
+    # the kernels round in another order (an element's FP32 forces, 2^-24 a
+    # rounding, about 20 of them); the records no more than a rounding on top
+    scale = np.linalg.norm(rd)
+    eb = np.linalg.norm(rb - rd) / scale
+    assert eb <= 2e-6 and np.linalg.norm(ra - rd) <= (2 * eb + 1e-7) * scale
+    ca, cb = a.counters(), b.counters()
+    assert cb["nr_active"] > 0 and abs(ca["nr_active"] - cb["nr_active"]) <= 1e-3 * cb["nr_active"]
+    # the surrogate takes a row per element and refuses a few rows, as before
+    import torch
+    from alya_sma_b200 import surrogate as S
+    net = S.Surrogate(seed=4)
+    net.fit_stats(torch.randn(256, S.NIN, device="cuda"), torch.randn(256, S.NOUT, device="cuda"))
+    if many:
+        a.set_surrogate(net)
+    else:
+        with pytest.raises(sma.SmaError, match="compact records"):
+            a.set_surrogate(net)
