@@ -352,9 +352,15 @@ __device__ __forceinline__ RMOut return_map(const MatC& m, double K, double G, d
 // residual at rounding level, which ends the reference's loop.  As the
 // reference: the activation tests (:351, :368), no step when the squared
 // first residual is at most 1e-8 (:403), the loading functions evaluated at
-// the unclamped xS, then the clamp (:484).  FP64, so the result is the
-// reference's to rounding.  Returns false, with nothing written, for both
-// transformations active and for a zero pivot; those take the iteration.
+// the unclamped xS, then the clamp (:484).  Returns false, with nothing
+// written, for both transformations active and for a zero pivot; those take
+// the iteration.  EXIT (FP64): so does a step beyond |dxS| = 1 (a pivot near
+// zero).  Up to there the residual it leaves ends the reference's loop (:454)
+// in units where rounding stays below that absolute test (closed_form_stops);
+// beyond, the loop may go on, and its further steps add the whole increment
+// again.  Tested before the division: evaluating the residual itself cost the
+// FP64 element loop 3.5 % (250 k elements) in registers.
+template <bool EXIT>
 __device__ __forceinline__ bool return_map_closed(const MatC& m, double K, double G, double G_1, double theta,
                                                   double e_n, double tmp, double& xS, double& F_AS,
                                                   double& F_SA, int& flag) {
@@ -382,7 +388,7 @@ __device__ __forceinline__ bool return_map_closed(const MatC& m, double K, doubl
     piv = (fsa - m.Rf_SA) - dot + x0 * G_1;
     other = fas - m.Rf_AS;
   }
-  if (piv == 0.0 || other == 0.0) return false;
+  if ((EXIT ? !(fabs(rhs) <= fabs(piv)) : piv == 0.0) || other == 0.0) return false;
   if (rhs * rhs > 1.0e-8) {
     const double x = x0 - rhs / piv;
     F_AS = loading(K, G, m.alfa, m.C_AS, m.eL, theta, e_n, tmp, x);
@@ -432,8 +438,9 @@ __device__ __forceinline__ int law160_from_A(const MatC& m, const T* A, double t
   bool done = false;
   // the FP32 form takes the closed form (element loop -1.3 % on the 2.0 M
   // cylinder, -4 % on the cantilever); the FP64 form keeps the reference's
-  // iteration, where the closed form's extra code cost it 3 % in spills
-  if constexpr (sizeof(T) == 4) done = return_map_closed(m, K, G, G_1, theta, e_n, tmp, xS, F_AS, F_SA, flag);
+  // iteration here, where the closed form's extra code cost it 3 % in spills
+  if constexpr (sizeof(T) == 4)
+    done = return_map_closed<false>(m, K, G, G_1, theta, e_n, tmp, xS, F_AS, F_SA, flag);
   if (!done) {
     RMOut r = return_map(m, K, G, G_1, theta, e_n, tmp, xS, F_AS, F_SA);
     xS = r.xS;

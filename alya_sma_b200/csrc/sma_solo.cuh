@@ -204,7 +204,7 @@ __device__ __forceinline__ bool law160_scalars(const MatC& m, T theta_t, T en2, 
   }
   const double theta = (double)theta_t, e_n = (double)en_t;
   flag = NR_NONE;
-  const bool ok = return_map_closed(m, K, G, G_1, theta, e_n, tmp, xS, F_AS, F_SA, flag);
+  const bool ok = return_map_closed<sizeof(T) == 8>(m, K, G, G_1, theta, e_n, tmp, xS, F_AS, F_SA, flag);
   pv = (T)(K * (theta - 3.0 * m.alfa * m.eL * xS));
   const T twoG = (T)(2.0 * G);
   kp = (en_t > T(2.220446049250313e-16)) ? twoG * (T(1) - (T)(m.eL * xS) * ie) : twoG;
