@@ -1131,6 +1131,7 @@ __global__ void __launch_bounds__(256) k_nodal(NodalArgs a) {
     }
   }
   if (MODE >= 1) count_warp(a.cnt, CNT_NONFINITE, valid && bad);
+  bool commit = blockIdx.x == 0;                                 // moves the time on; nothing above reads what it writes
   if (ENERGY && MODE >= 1) {
     // fixed-order sums (warp butterfly, then the block's 8 warps in order)
     // into one partial per block, so the balance is bitwise reproducible
@@ -1162,8 +1163,9 @@ __global__ void __launch_bounds__(256) k_nodal(NodalArgs a) {
       energy_finalize(a.en_step, (int)gridDim.x, a.en_tot, a.en_hist, a.en_row, a.en_max_rows);
       if (threadIdx.x == 0) *a.en_ticket = 0u;
     }
+    commit = last;                                               // but the work terms, which read ts.load
   }
-  if (MODE != 2 && blockIdx.x == 0 && threadIdx.x == 0) {
+  if (MODE != 2 && commit && threadIdx.x == 0) {
     a.ts->cutim = a.ts->nx_cutim;
     a.ts->load = a.ts->nx_load;
   }

@@ -156,6 +156,37 @@ def test_energy_balance_matches_restatement(oracle, canti, alpha, scheme):
     assert ref[-1, 1] > 0.0                                   # the traction did work
 
 
+@pytest.mark.parametrize("alpha,scheme", [(0.0, "cd"), (1.0e5, "cd"), (0.0, "tw")])
+def test_energy_work_of_more_nodes_than_fit_at_once(alpha, scheme):
+    """A load that changes by a tenth per step on every node of a mesh whose
+    nodal update takes more than one wave of blocks: each block's work term has
+    its own step's load factor, in a chunk of steps as in single ones (whose
+    update does not move the time on)."""
+    n = 68                                                     # 328,509 nodes; a wave holds 303,104 at most
+    coord, lnods = P.structured_box(n, n, n, float(n), float(n), float(n), 0.05, 3)
+    npo = len(coord)
+    props, densi = P.nitinol_props(**P.NITI)[None, :], np.array([P.NITI_DENSITY])
+    dt = 0.5 * P.critical_dt(coord, lnods, props, densi)
+    fixno = np.zeros((npo, 3), np.int32)
+    fixno[P.face_nodes(coord, 0, 0.0)] = 1
+    p = P.Problem(coord=coord, lnods=lnods, props=props, e_mart=np.zeros(1), densi=densi, fixno=fixno,
+                  bcfun=np.full(npo, -1, np.int32), fun_npts=np.array([3], np.int32),
+                  fun_smooth=np.array([0], np.int32), fun_tab=P.smooth_cycle_table(20 * dt, 1.0),
+                  fext=np.random.default_rng(1).normal(size=(npo, 3)), load_fun=0, dtime=dt, nsteps=20,
+                  dampi=np.array([[alpha, 0.0]]))
+    h = []
+    for chunk in (12, 1):
+        s = sma.ExplicitSolid(p, precision="fp64", scheme=scheme)
+        s.set_energy(True, 12)
+        for _ in range(12 // chunk):
+            s.step(chunk)
+        h.append(s.energy()[1])
+        s.close()
+    assert h[0].shape == h[1].shape == (12, 5) and h[1][-1, 1] > 0.0
+    # sums of 10^6 terms of either sign, the residual's atomics in any order
+    assert np.abs(h[0] - h[1]).max() <= 1e-9 * np.abs(h[1]).max()
+
+
 def test_reaction_witness(oracle, canti):
     """Residual witnesses on the clamped face are the reactions frxid_sld:
     after the element loop they equal the oracle's rhsid there."""
