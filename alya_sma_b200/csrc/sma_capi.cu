@@ -327,7 +327,6 @@ struct sma_ctx {
   double dtcri = 0.0;
   double dtime = 0.0;
   bool has_load = false;
-  double grav[3] = {0, 0, 0};
   // graphs: chunk of steps starting at state parity 0 / 1
   cudaGraphExec_t gexec[2] = {nullptr, nullptr};
   int gchunk = 0;
@@ -474,10 +473,6 @@ ElemArgs<T> elem_args(sma_ctx* c, int beg, int end, bool advance, bool stepping 
   a.matx = (const T*)c->d_matx;
   // one wave of the one-tile kernel: every SM's resident blocks of block / 8 elements
   a.pf_ahead = (c->variant == SMA_VARIANT_PIPE) ? 0 : (int64_t)c->nsm * c->resident * (c->block / 8);
-  a.grav[0] = c->grav[0];
-  a.grav[1] = c->grav[1];
-  a.grav[2] = c->grav[2];
-  a.has_grav = (c->grav[0] != 0.0 || c->grav[1] != 0.0 || c->grav[2] != 0.0);
   return a;
 }
 
@@ -538,6 +533,7 @@ ElemKernel<T> solo_kernel(const sma_ctx* c) {
 // 19.6 k 14.6 / 19.0 us.  Above it they fall behind: 32 k 17.0 / 25.5 us
 // against 14.9 / 18.9, 250 k 78 / 146 us against 52 / 90.
 int solo_min(const sma_ctx* c) { return 128 * c->nsm; }
+bool takes_solo(const sma_ctx* c, int nelem) { return c->solo && c->solo_block && nelem >= solo_min(c); }
 
 // a kernel of the step, resident before its predecessor on the stream has
 // finished (programmatic dependent launch; the kernels wait for it before
@@ -558,12 +554,16 @@ cudaError_t launch_step(sma_ctx* c, void (*k)(P...), unsigned grid, int block, s
 }
 
 // one element range [beg, end), by the thread-per-element kernel where the
-// context has it and the range fills the GPU with it, else 8 lanes per element
+// context has it and the range fills the GPU with it, else 8 lanes per element.
+// beside: the side pass adds the damping force (damp_beside), which the 8-lane
+// kernel would add itself
 template <typename T>
 int32_t launch_range_t(sma_ctx* c, int beg, int end, bool advance, bool stepping, bool beside = false) {
   if (end <= beg) return SMA_OK;
   ElemArgs<T> a = elem_args<T>(c, beg, end, advance, stepping);
-  if (c->solo && c->solo_block && end - beg >= solo_min(c) && !a.has_grav && (!c->damp || beside)) {
+  const bool solo = takes_solo(c, end - beg) && (!c->damp || beside);
+  if (beside && !solo) return fail(SMA_ERR_STATE, "damping beside an element loop that folds it in");
+  if (solo) {
     const int block = c->solo_block;
     a.pf_ahead = (int64_t)c->nsm * solo_min_blocks<T>() * SOLO_BLOCK;      // one resident wave
     CU(launch_step(c, solo_kernel<T>(c), (unsigned)ceil_div(end - beg, block) + (a.ts ? 1 : 0), block,
@@ -879,7 +879,7 @@ int32_t launch_rayleigh(sma_ctx* c, const double* vel, cudaStream_t s, bool forc
 // 48.0 / 38.8 us, with the energy balance 60.2 / 46.4, FP32 30.9 / 26.9; 250 k
 // cylinder FP32 121 / 110; below two warps per scheduler the second launch
 // costs more than it gives: 25.6 k FP32 15.4 / 17.0).
-bool damp_beside(const sma_ctx* c) { return c->damp && c->solo && c->plan_end.empty(); }
+bool damp_beside(const sma_ctx* c) { return c->damp && c->plan_end.empty() && takes_solo(c, c->nelem); }
 bool side_rayleigh(const sma_ctx* c) { return c->damp && (c->energy || damp_beside(c)); }
 int32_t fork_rayleigh(sma_ctx* c) {
   CU(cudaEventRecord(c->ev_side[0], c->stream));
@@ -2205,7 +2205,6 @@ int32_t noalloc_run(unsigned char* base, int32_t nelem, int32_t npoin, const int
   a.tiled = 0;
   a.beg = 0;
   a.end = nelem;
-  a.has_grav = 0;
   a.vel = nullptr;
   // the one-material narrow instance at one-warp blocks, as a context
   // with one material runs it by default

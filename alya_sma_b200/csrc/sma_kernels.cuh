@@ -157,8 +157,6 @@ struct ElemArgs {
   int64_t npad, sst;
   int tiled;                   // state layout (state_index)
   int32_t beg, end;            // element range of this launch
-  double grav[3];              // rho-scaled body force per unit mass (elfext)
-  int has_grav;
   const double* vel;           // SoA [3][npad] velocity for Rayleigh alpha, or null
   MatC mat0;                   // the material when lmate is null (kernel-parameter space);
                                // with compact records the values every element shares
@@ -391,7 +389,7 @@ __device__ __forceinline__ T gp_kinematics(const T* nsm, int g, T* Ji, T* H, T* 
 
 // Phase 2 of a tile once the Kirchhoff stress tau of this lane's Gauss point
 // is known: the force operator Q = vol tau (F J)^-T in shared memory, then
-// lane = node a sums f_a = -sum_g Q_g dN_a(g) (+ the body force) and
+// lane = node a sums f_a = -sum_g Q_g dN_a(g) (+ the damping force) and
 // scatters it (FP64 atomics or read-modify-write).  Jc = 8 F J.  Returns
 // det(8 F J).
 template <typename T, bool ATOMIC, bool DAMP>
@@ -411,32 +409,24 @@ __device__ __forceinline__ T tile_forces(const ElemArgs<T>& a, const T* tab, T* 
     q[3 + m] = t01 * B[3 * m + 0] + t11 * B[3 * m + 1] + t12 * B[3 * m + 2];
     q[6 + m] = t02 * B[3 * m + 0] + t12 * B[3 * m + 1] + t22 * B[3 * m + 2];
   }
-  // body force of the Gauss point, dV rho (g - alpha v(g)): gravity
-  // (elfext) and the Rayleigh alpha term (elrayl_alpha, sld_elmmat.f90:159-
-  // 164) with v(g) = sum_b N_b(g) v_b from the element's lanes by shuffle
-  const bool body = DAMP || a.has_grav;
-  if (body) {
-    const T rho = (T)mat.densi;
-    T b0 = rho * (T)a.grav[0], b1 = rho * (T)a.grav[1], b2 = rho * (T)a.grav[2];
-    if constexpr (DAMP) {
-      T N[8], dN[24];
-      hex8_gp<T>(lane8, N, dN);
-      const int src = (threadIdx.x & 31) & ~7;
-      T v0 = T(0), v1 = T(0), v2 = T(0);
+  // Rayleigh alpha force of the Gauss point, -dV rho alpha v(g) (elrayl_alpha,
+  // sld_elmmat.f90:159-164), with v(g) = sum_b N_b(g) v_b from the element's
+  // lanes by shuffle
+  if constexpr (DAMP) {
+    T N[8], dN[24];
+    hex8_gp<T>(lane8, N, dN);
+    const int src = (threadIdx.x & 31) & ~7;
+    T v0 = T(0), v1 = T(0), v2 = T(0);
 #pragma unroll
-      for (int b = 0; b < 8; ++b) {
-        v0 += N[b] * __shfl_sync(0xffffffffu, Vn[0], src + b);
-        v1 += N[b] * __shfl_sync(0xffffffffu, Vn[1], src + b);
-        v2 += N[b] * __shfl_sync(0xffffffffu, Vn[2], src + b);
-      }
-      const T ra = rho * (T)mat.ray_a;
-      b0 -= ra * v0;
-      b1 -= ra * v1;
-      b2 -= ra * v2;
+    for (int b = 0; b < 8; ++b) {
+      v0 += N[b] * __shfl_sync(0xffffffffu, Vn[0], src + b);
+      v1 += N[b] * __shfl_sync(0xffffffffu, Vn[1], src + b);
+      v2 += N[b] * __shfl_sync(0xffffffffu, Vn[2], src + b);
     }
-    q[9] = vol * b0;
-    q[10] = vol * b1;
-    q[11] = vol * b2;
+    const T ra = (T)mat.densi * (T)mat.ray_a;
+    q[9] = -vol * (ra * v0);
+    q[10] = -vol * (ra * v1);
+    q[11] = -vol * (ra * v2);
   }
   __syncwarp();
 
@@ -452,7 +442,7 @@ __device__ __forceinline__ T tile_forces(const ElemArgs<T>& a, const T* tab, T* 
     f0 -= qg[0] * dn[0] + qg[1] * dn[1] + qg[2] * dn[2];
     f1 -= qg[3] * dn[0] + qg[4] * dn[1] + qg[5] * dn[2];
     f2 -= qg[6] * dn[0] + qg[7] * dn[1] + qg[8] * dn[2];
-    if (body) {
+    if constexpr (DAMP) {
       f0 += dn[3] * qg[9];
       f1 += dn[3] * qg[10];
       f2 += dn[3] * qg[11];

@@ -193,6 +193,37 @@ def test_damped_steps_equal_the_8_lane_kernel(precision, scheme, energy):
             assert abs(ta[k] - tb[k]) <= 10 * tol * abs(tb[k]), k
 
 
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+def test_one_damping_force_under_plans_and_host_driven_steps(precision):
+    """The damping force is added once, whether the pass beside the loop or
+    the 8-lane kernel adds it: launch plans, element ranges and whole steps of
+    one context."""
+    prob = _damped_mesh()
+    u = P.prestrain(prob, 0.01)
+    v = 1.0e3 * np.random.default_rng(1).normal(size=u.shape)
+    a, b = _pair(prob, precision)
+    lib, n = sma.lib(), prob.nelem
+    for s in (a, b):
+        s.set("displ", u)
+        s.set("veloc", v)
+    a.set_launch_plan([20_011, n], [64, 128])
+    for s in (a, b):
+        s.step(4)
+    a.set_launch_plan([], [])
+    for s in (a, b):
+        s.step(4)
+        assert lib.sma_step_prologue(s._ctx) == 0
+        for cut in (0, 19_999, n):                          # whole, and in two ranges
+            for beg, end in zip((0, cut), (cut, n)):
+                if end > beg:
+                    assert lib.sma_step_elements_range(s._ctx, beg, end, int(beg == 0), int(end == n)) == 0
+            assert lib.sma_step_nodes(s._ctx, int(cut == n)) == 0
+    tol = 1e-10 if precision == "fp64" else 1e-4
+    for f in ("displ", "veloc"):
+        x, y = a.get(f), b.get(f)
+        assert np.linalg.norm(x - y) <= tol * np.linalg.norm(y), f
+
+
 @pytest.mark.parametrize("timed", [False, True])
 @pytest.mark.parametrize("scheme,energy", [("cd", False), ("cd", True), ("tw", False)])
 def test_residual_witnesses_hold_the_damping_force(scheme, energy, timed):
