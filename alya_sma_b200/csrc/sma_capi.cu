@@ -737,8 +737,15 @@ int32_t launch_element_range_t(sma_ctx* c, int beg, int end) {
 // slab touches them).  Meshes numbered with locality (structured, O-grid,
 // concatenated specimens) give growing prefixes, so the copies in and out
 // overlap the element work; a mesh without it degrades to need = npoin.
+// Slabs hold at least 16,384 elements, or as many as take the
+// thread-per-element kernel where the context's element loop does (51,200
+// elements in two slabs instead of three with 8 lanes per element: FP32 107 ->
+// 96 us, FP64 126 -> 107; 100,000 in five instead of six: 171 -> 166, 202 -> 178),
+// but two slabs from 32,768 on, since one overlaps no copy (33,858: 92 us with
+// two, 99 with one).
 void plan_pipeline(sma_ctx* c, const int32_t* ln) {
-  const int K = (int)std::min<int64_t>(8, std::max<int64_t>(1, c->nelem / 16384));
+  const int64_t small = c->nelem / 16384, solo = c->solo && !c->damp ? c->nelem / solo_min(c) : small;
+  const int K = (int)std::min<int64_t>(8, std::max<int64_t>({1, solo, std::min<int64_t>(2, small)}));
   c->pl_e.assign(K + 1, 0);
   c->pl_need.assign(K, 0);
   c->pl_final.assign(K, 0);
@@ -1192,17 +1199,6 @@ int32_t sma_ctx_create(const sma_mesh_desc* mesh, const sma_material_desc* mat,
     std::memcpy(&lnods_i[8 * (size_t)e], mesh->lnods + 8 * (int64_t)c->perm[e], 8 * sizeof(int32_t));
   TRY(dalloc(&c->d_lnods, lnods_i.size() * sizeof(int32_t)));
   TRYCU(cudaMemcpy(c->d_lnods, lnods_i.data(), lnods_i.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
-  if (c->scatter == SMA_SCATTER_ATOMIC) {
-    plan_pipeline(c, lnods_i.data());
-    if (c->pl_need.size() >= 2) {
-      TRYCU(cudaStreamCreateWithFlags(&c->s_h2d, cudaStreamNonBlocking));
-      TRYCU(cudaStreamCreateWithFlags(&c->s_d2h, cudaStreamNonBlocking));
-      c->pl_ev.resize(2 * c->pl_need.size() + 1, nullptr);
-      for (cudaEvent_t& e : c->pl_ev) TRYCU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    } else {
-      c->pl_need.clear();                  // one slab: the serial path
-    }
-  }
   TRY(dalloc(&c->d_perm, c->perm.size() * sizeof(int32_t)));
   TRYCU(cudaMemcpy(c->d_perm, c->perm.data(), c->perm.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
   if (mesh->lmate && c->nmate > 1) {
@@ -1237,6 +1233,17 @@ int32_t sma_ctx_create(const sma_mesh_desc* mesh, const sma_material_desc* mat,
   if (c->solo) {
     if (run->block) c->solo_block = run->block;
     c->sst = 8 * (ceil_div(c->nelem, 32) * 32);                 // whole tiles: 3 sst values
+  }
+  if (c->scatter == SMA_SCATTER_ATOMIC) {
+    plan_pipeline(c, lnods_i.data());
+    if (c->pl_need.size() >= 2) {
+      TRYCU(cudaStreamCreateWithFlags(&c->s_h2d, cudaStreamNonBlocking));
+      TRYCU(cudaStreamCreateWithFlags(&c->s_d2h, cudaStreamNonBlocking));
+      c->pl_ev.resize(2 * c->pl_need.size() + 1, nullptr);
+      for (cudaEvent_t& e : c->pl_ev) TRYCU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    } else {
+      c->pl_need.clear();                  // one slab: the serial path
+    }
   }
   // Compact per-element records when the materials differ only in what the
   // record holds (moduli, eL, thresholds; the temperature rides along) and

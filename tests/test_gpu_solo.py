@@ -109,6 +109,29 @@ def test_points_outside_the_short_forms(kind, precision):
     assert np.array_equal(np.isnan(a.assemble(v)["rhsid"]), np.isnan(b.assemble(v)["rhsid"]))
 
 
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("nx,slabs", [(57, 1), (97, 2), (113, 2), (146, 2), (176, 3), (500, 8)])
+def test_element_loop_on_host_arrays_in_slabs(nx, slabs, precision):
+    """The pipelined element loop on host arrays: slabs of the thread-per-element
+    kernel, except the two that overlap the copies of a mesh too small for two
+    of them; the same residual as one serial call of the 8-lane kernel."""
+    base = _mesh("one")
+    coord, lnods = P.structured_box(nx, 17, 20, float(nx), 17.0, 20.0, 0.1, 5)
+    npo = len(coord)
+    prob = dataclasses.replace(base, coord=coord, lnods=lnods, fixno=np.zeros((npo, 3), np.int32),
+                               bcfun=np.full(npo, -1, np.int32),
+                               fext=P.face_load(coord, lnods, 0, float(nx), (1.0, 0.0, 0.0)))
+    u = P.prestrain(prob, 0.01) + 1e-3 * np.random.default_rng(2).normal(size=coord.shape)
+    a, b = _pair(prob, precision)
+    n0 = a.kernel_launches
+    ra = a.assemble(u, fext_scale=0.5, want_all=False)["rhsid"]
+    # per slab: displacement in, elements, finished residual rows out (one: displacement, load, elements, residual)
+    assert a.kernel_launches - n0 == (3 * slabs if slabs > 1 else 4)
+    rb = b.assemble(u, fext_scale=0.5)["rhsid"]
+    assert np.linalg.norm(ra - rb) <= (1e-12 if precision == "fp64" else 2e-6) * np.linalg.norm(rb)
+    assert np.linalg.norm(a.state - b.state) <= (1e-12 if precision == "fp64" else 1e-5) * np.linalg.norm(b.state)
+
+
 def test_ranges_checkpoints_and_plans_share_the_state(tmp_path):
     """One context's element ranges go to either kernel (a launch plan with
     narrow and wide blocks, slabs below the threshold), and a checkpoint moves
