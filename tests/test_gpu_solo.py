@@ -132,24 +132,51 @@ def test_element_loop_on_host_arrays_in_slabs(nx, slabs, precision):
     assert np.linalg.norm(a.state - b.state) <= (1e-12 if precision == "fp64" else 1e-5) * np.linalg.norm(b.state)
 
 
-def test_ranges_checkpoints_and_plans_share_the_state(tmp_path):
+def _close(a, b, tol):
+    for f in ("displ", "veloc"):
+        x, y = a.get(f), b.get(f)
+        assert np.linalg.norm(x - y) <= tol * np.linalg.norm(y), f
+    x, y = a.state, b.state
+    assert np.linalg.norm(x - y) <= 10 * tol * np.linalg.norm(y)
+    ca, cb = a.counters(reset=True), b.counters(reset=True)
+    # as in test_steps_equal_the_8_lane_kernel
+    assert cb["nr_active"] > 0 and abs(ca["nr_active"] - cb["nr_active"]) <= 0.1 * cb["nr_active"]
+    assert ca["neg_det"] == cb["neg_det"] == 0
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("kind", ["one", "compact", "table"])
+def test_ranges_checkpoints_and_plans_share_the_state(tmp_path, kind, precision):
     """One context's element ranges go to either kernel (a launch plan with
-    narrow and wide blocks, slabs below the threshold), and a checkpoint moves
-    between state layouts."""
-    prob = dataclasses.replace(_mesh("one"))
+    narrow and wide blocks, element ranges below and above the threshold that
+    start inside a state tile), and a checkpoint moves between state layouts."""
+    prob = _mesh(kind)
     u = P.prestrain(prob, 0.01)
-    a, b = _pair(prob, "fp64")
-    a.set_launch_plan([19_001, prob.nelem], [32, 128])
+    a, b = _pair(prob, precision)
+    lib, n = sma.lib(), prob.nelem
+    tol = 1e-11 if precision == "fp64" else 2e-5
     for s in (a, b):
         s.set("displ", u)
-        s.step(5)
+    for ends, blocks in (([19_001, n], [32, 128]), ([1_003, n], [256, 64])):
+        a.set_launch_plan(ends, blocks)
+        for s in (a, b):
+            s.step(5)
+        _close(a, b, tol)
     a.set_launch_plan([], [])
+    for s in (a, b):
+        assert lib.sma_step_prologue(s._ctx) == 0
+        for k in range(5):
+            for beg, end in ((0, 1_003), (1_003, n)):
+                assert lib.sma_step_elements_range(s._ctx, beg, end, int(beg == 0), int(end == n)) == 0
+            assert lib.sma_step_nodes(s._ctx, int(k == 4)) == 0
+    _close(a, b, tol)
     a.save(str(tmp_path / "c"))
     b.load(str(tmp_path / "c"))
     assert np.array_equal(a.state, b.state)
-    a.step(5)
-    b.step(5)
-    assert np.abs(a.get("displ") - b.get("displ")).max() <= 1e-12 * np.abs(b.get("displ")).max()
+    a.counters(reset=True), b.counters(reset=True)
+    for s in (a, b):
+        s.step(5)
+    _close(a, b, tol)
 
 
 def test_surrogate_and_postprocessing_read_the_tiled_state():
