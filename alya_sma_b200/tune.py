@@ -1,10 +1,10 @@
-"""Autotuner for the element loop: threads per block (the element tile: 8
-Gauss-point lanes per element, so block/8 elements per tile), the
-scatter-add (FP64 atomics or colour blocks) and the element kernel (one
-tile per block, or persistent blocks with the next tile's gather in
-flight), picked by timing each
-candidate on the caller's own mesh with the device phase timers
-(sma_set_timing) and cached per (precision, scheme, size bucket).
+"""Autotuner for the element loop: threads per block, the scatter-add (FP64
+atomics or colour blocks) and the element kernel (the library's own choice,
+which is one thread per element on large meshes; 8 Gauss-point lanes per
+element, one tile of block/8 elements per block; or persistent blocks with the
+next tile's gather in flight), picked by timing each candidate on the caller's
+own mesh with the device phase timers (sma_set_timing) and cached per
+precision, scheme, material layout, damping and size bucket.
 
 The size bucket is the element count rounded to a power of two, so a cached
 choice carries over to meshes of similar size (ensemble members, refinements).
@@ -15,9 +15,15 @@ import json
 import math
 import os
 
-CANDIDATES = ((32, "atomic", "plain"), (64, "atomic", "plain"), (128, "atomic", "plain"),
+# block 0: the library's default.  "auto" with a block of up to 64 threads may
+# take one thread per element; the other variants are 8 lanes per element
+CANDIDATES = ((0, "atomic", "auto"), (32, "atomic", "auto"),
+              (32, "atomic", "plain"), (64, "atomic", "plain"), (128, "atomic", "plain"),
               (256, "atomic", "plain"), (128, "atomic", "pipe"), (256, "atomic", "pipe"),
               (64, "color", "plain"), (256, "color", "pipe"))
+
+# raised with the kernels or the candidates: choices cached before are not used
+GENERATION = 2
 
 
 def cache_path() -> str:
@@ -30,8 +36,12 @@ def bucket(nelem: int) -> int:
     return 1 << max(0, int(round(math.log2(max(1, nelem)))))
 
 
-def _key(precision, scheme, nelem):
-    return f"{precision}/{scheme}/{bucket(nelem)}"
+def _key(precision, scheme, prob):
+    """What decides which kernels a mesh can take and how they compare."""
+    nmate = len(prob.props) if prob.lmate is not None else 1
+    mats = "one" if nmate == 1 else ("many" if 4 * nmate >= prob.nelem else "few")
+    damped = prob.dampi is not None and bool((prob.dampi[:, 0] > 0.0).any())
+    return f"{GENERATION}/{precision}/{scheme}/{mats}{'/damped' if damped else ''}/{bucket(prob.nelem)}"
 
 
 def load_cache(path=None) -> dict:
@@ -59,7 +69,7 @@ def tune(prob, precision="fp32", scheme="cd", candidates=CANDIDATES, steps=20, w
     state (displ, if given) with per-phase device timing; the fastest whole
     step wins."""
     from . import ExplicitSolid
-    key = _key(precision, scheme, prob.nelem)
+    key = _key(precision, scheme, prob)
     cache = load_cache(path) if use_cache else {}
     if use_cache and key in cache:
         return cache[key]
@@ -90,7 +100,7 @@ def tune(prob, precision="fp32", scheme="cd", candidates=CANDIDATES, steps=20, w
 
 
 def autotuned(prob, precision="fp32", scheme="cd", device=0, **kw):
-    """An ExplicitSolid built with the tuned block size and scatter."""
+    """An ExplicitSolid built with the tuned block size, scatter and kernel."""
     from . import ExplicitSolid
     r = tune(prob, precision=precision, scheme=scheme, device=device, **kw)
     return ExplicitSolid(prob, precision=precision, scatter=r["scatter"], block=r["block"],
@@ -134,7 +144,7 @@ def tune_buckets(prob, precision="fp32", candidates=(32, 64, 128, 256), steps=10
         s.set_timing(False)
         return t["step"][0] / steps
 
-    default_block = 128 if len(prob.props) > 1 else 32
+    default_block = s.launch_info()["block"]
     pick = [default_block] * len(ends)
     trials = {}
     for _ in range(rounds):

@@ -136,6 +136,32 @@ def test_autotuner_picks_and_caches(tmp_path, monkeypatch):
     assert s.counters()["nonfinite"] == 0
 
 
+def test_autotuner_finds_the_thread_per_element_kernel(tmp_path, monkeypatch):
+    """102,400 elements: the library's own choice is among the candidates and,
+    one thread per element, faster than 8 lanes by far more than the timings
+    differ; a default block for buckets is the context's own."""
+    monkeypatch.setenv("ALYA_SMA_CACHE", str(tmp_path))
+    coord, lnods = P.structured_box(100, 32, 32, 100.0, 32.0, 32.0, 0.05, 5)
+    npo = len(coord)
+    props, densi = P.nitinol_props(**P.NITI)[None, :], np.array([P.NITI_DENSITY])
+    fixno = np.zeros((npo, 3), np.int32)
+    fixno[P.face_nodes(coord, 0, 0.0)] = 1
+    dt = 0.5 * P.critical_dt(coord, lnods, props, densi)
+    p = P.Problem(coord=coord, lnods=lnods, props=props, e_mart=np.array([P.NITI_E_MART]), densi=densi, fixno=fixno,
+                  bcfun=np.full(npo, -1, np.int32), fun_npts=np.array([3], np.int32),
+                  fun_smooth=np.array([1], np.int32), fun_tab=P.smooth_cycle_table(1000 * dt, 700.0),
+                  fext=P.face_load(coord, lnods, 0, 100.0, (1.0, 0.0, 0.0)), load_fun=0, dtime=dt, nsteps=1000)
+    u = P.prestrain(p, 0.01)
+    r = tune.tune(p, precision="fp32", steps=20, warmup=3, displ=u)
+    assert r["variant"] == "auto" and {"0/atomic/auto", "32/atomic/auto"} <= set(r["trials"])
+    lanes8 = min(t["element_ms"] for k, t in r["trials"].items() if not k.endswith("/auto"))
+    assert min(t["element_ms"] for k, t in r["trials"].items() if k.endswith("/auto")) < 0.9 * lanes8
+    assert tune.autotuned(p, precision="fp32", displ=u).launch_info()["block"] in (32, 64)
+    e = P.ensemble(nspec=24, nsteps=100)                    # a launch plan per size bucket
+    t = tune.tune_buckets(e, precision="fp32", steps=3, warmup=1)
+    assert t["default_block"] == sma.ExplicitSolid(e, precision="fp32").launch_info()["block"] == 64
+
+
 @pytest.mark.parametrize("name", ["cylinder", "bar"])
 def test_prestrained_start_is_physical(name):
     """The bench's prestrained start on a mesh whose far end is held by a
