@@ -1155,8 +1155,9 @@ int32_t sma_ctx_create(const sma_mesh_desc* mesh, const sma_material_desc* mat,
   TRYCU(cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking));
   c->prec = run->precision;
   c->scatter = (run->scatter == SMA_SCATTER_COLOR) ? SMA_SCATTER_COLOR : SMA_SCATTER_ATOMIC;
-  // default variant, measured on B200 (cantilever 640k and cylinder 2.0M
-  // elements, fixed step windows): the one-tile kernel in both precisions;
+  // default variant where the element loop takes 8 lanes per element (large
+  // meshes: one thread, below), measured on B200 (cantilever 640k and cylinder
+  // 2.0M elements, fixed step windows): the one-tile kernel in both precisions;
   // with the register caps of the element kernels the pipelined variant
   // spills and is 10-50 % slower
   if (run->variant < SMA_VARIANT_AUTO || run->variant > SMA_VARIANT_TABLE)

@@ -203,8 +203,21 @@ def measured_peaks():
 
 
 KERNEL_SOURCES = ("alya_sma_b200/csrc/sma_capi.cu", "alya_sma_b200/csrc/sma_kernels.cuh",
-                  "alya_sma_b200/csrc/sma_law.cuh", "alya_sma_b200/csrc/sma_surrogate.cuh",
-                  "alya_sma_b200/csrc/sma_surrogate_elem.cuh", "alya_sma_b200/build.py")
+                  "alya_sma_b200/csrc/sma_law.cuh", "alya_sma_b200/csrc/sma_solo.cuh",
+                  "alya_sma_b200/csrc/sma_surrogate.cuh", "alya_sma_b200/csrc/sma_surrogate_elem.cuh",
+                  "alya_sma_b200/build.py")
+
+
+def element_kernel(info, precision, nelem, block=0, scatter="atomic", variant="auto"):
+    """Name of the kernel a context's whole element launch runs, from its
+    arguments and launch_info(): one thread per element (default block 64),
+    8 lanes (default 32 or 128), persistent, or the surrogate's."""
+    if precision == "surrogate":
+        return "k_element_sur"
+    if info["variant"] == "pipe":
+        return "k_element_pipe"
+    solo = info["block"] == 64 if not block else block <= 64 and nelem >= 128 * 148
+    return "k_element_solo" if variant == "auto" and scatter == "atomic" and solo else "k_element"
 
 
 def kernel_source_hash():
@@ -621,7 +634,8 @@ def run_partitioned(args, rank, world, local):
     achieved = alg / (el_ms / 1e3) / 1e9
     prof = load_profile(args.precision, args.workload, q.nelem) if (world == 1 and args.div == 1
                                                                        and not args.layers) else None
-    roofline = {"bound": "hbm", "kernel": "k_element", "achieved": round(achieved, 1), "peak": peak,
+    kernel = element_kernel(part.launch_info(), args.precision, q.nelem, args.block, args.scatter)
+    roofline = {"bound": "hbm", "kernel": kernel, "achieved": round(achieved, 1), "peak": peak,
                 "peak_kind": peak_kind, "unit": "GB/s", "frac": round(achieved / peak, 4),
                 "traffic": prof["traffic"] if prof else None, "algorithmic_bytes_per_launch": alg,
                 "launch_ms": round(el_ms, 4), "exchange_ms": round(ex_ms, 4), "nodal_launch_ms": round(nd_ms, 4),
@@ -773,8 +787,9 @@ def main():
     alg = algorithmic_bytes(prob, args.precision)
     achieved = alg / (el_ms / 1e3) / 1e9
     prof = load_profile(args.precision, args.workload, nelem) if (args.div == 1 and not args.layers) else None
-    roofline = {"bound": "hbm", "kernel": "k_element", "achieved": round(achieved, 1),
-                "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
+    roofline = {"bound": "hbm",
+                "kernel": element_kernel(launch_info, args.precision, nelem, block, scatter, variant),
+                "achieved": round(achieved, 1), "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
                 "frac": round(achieved / peak, 4), "traffic": prof["traffic"] if prof else None,
                 "algorithmic_bytes_per_launch": alg,
                 "algorithmic_bytes_per_gauss_point": round(alg / ngp, 1),

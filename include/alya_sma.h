@@ -111,7 +111,8 @@ typedef struct {
 } sma_run_desc;
 
 /* element-loop kernels */
-#define SMA_VARIANT_AUTO    0   /* PLAIN in both precisions (measured on B200)                */
+#define SMA_VARIANT_AUTO    0   /* one thread per element on large meshes (atomic scatter,    */
+                                /* blocks of up to 64 threads), else PLAIN                    */
 #define SMA_VARIANT_PIPE    1   /* persistent blocks, next tile's gather in flight (cp.async) */
 #define SMA_VARIANT_PLAIN   2   /* one tile per block; per-element materials that differ only */
                                 /* in E_A, E_M, eL and thresholds as compact 8-word records   */
