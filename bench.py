@@ -840,7 +840,10 @@ def main():
             spread.append(su)
         extras["error_vs_fp64"] = compare_forms(prob, solid, s64, wsteps + args.steps, spread)
         if args.surrogate:
-            extras["surrogate"] = surrogate_leg(args, prob, u0, s64, v64, value / world, wsteps, local, spread)
+            try:
+                extras["surrogate"] = surrogate_leg(args, prob, u0, s64, v64, value / world, wsteps, local, spread)
+            except sma.SmaError as e:              # a mesh it does not take (the ensemble's few materials)
+                extras["surrogate"] = {"unavailable": str(e)}
         for su in spread:
             su.close()
         s64.close()
