@@ -304,11 +304,13 @@ static __global__ void k_sur_generate(GenArgs g) {
 // a thread) until the block is done, so no sum goes through memory.  silu and
 // its derivative share one sigmoid per activation, the derivative kept in
 // FP16 pairs in registers until the backward pass.
-// Bound: the mma.sync pipe and its shared-memory operands.  Before, a warp
-// added each 32 samples' gradient to a shared copy by 14,600 atomics, which
-// FP32 shared atomics make compare-and-swap loops, with 4 warps per SM:
-// 1,009 us for the gradient of 262,144 samples, 202 us now, and no less exact
-// (2.1e-4 of the FP64 gradient, 2.4e-4 before).
+// Bound: latency, with 8 warps per SM (255 registers): issue 28 %, mma.sync
+// pipe 25 %; the stalls are the turn's inputs and targets from memory, fixed
+// latency, ldmatrix and the five block barriers.  Before, a warp added each 32
+// samples' gradient to a shared copy by 14,600 atomics, which FP32 shared
+// atomics make compare-and-swap loops, with 4 warps per SM: 1,009 us for the
+// gradient of 262,144 samples, 202 us now, and no less exact (2.1e-4 of the
+// FP64 gradient, 2.4e-4 before).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void mma16816(float* d, const uint32_t* a, const uint32_t* b) {
   asm volatile(
